@@ -143,7 +143,7 @@ int sfh_cg_solve(sfh_ctx* ctx, const double* phi, double* X, double tol, int max
 /* The schedule of the context's mixed-precision solves (sfh_cg_solve, the
  * trajectory's solves), as sfh_batch_set_schedule: RHS-block width, tiles per
  * block, link staging 0..7 (3: the whole solve in one persistent launch).
- * Default 0, 0, 0; the FP64 CG keeps its own (default tiles per block).  No
+ * Default 0, 0, 0 (also the FP64 CG's, whatever is set here).  No
  * counterpart in the reference. */
 int sfh_set_schedule(sfh_ctx* ctx, int width, int tiles_per_block, int stage_links);
 
@@ -336,13 +336,18 @@ int sfh_batch_get_hop_widths(sfh_batch* batch, int* hop1_width, int* hop2_width)
  * (1, 2, 4, 8; FP64: 1, 2), tiles-per-block count (1, 2, 4) and link staging
  * (0 to 7 as below; FP64: 0; 6 for FP16 only), and for the lane-list stages
  * (4 to 7) also hop widths 4 and 2, on the batch's current inputs and keep
- * the fastest.
+ * the fastest; where the dataflow launch of small batches is faster still, it
+ * runs the solves until a schedule is set.
  * The schedule never changes the results.  No counterpart in the reference
  * (its solver has no schedule). */
 int sfh_batch_autotune(sfh_batch* batch, int probe_iters, int* best_width);
 /* The schedule directly: RHS-block width (0 = automatic), 256-site tiles per
  * block of the iteration kernels (0 = 2, or 1 where two would give the first
- * hop fewer than four work items per SM), and the hop kernels' link staging:
+ * hop fewer than four work items per SM), and the hop kernels' link staging
+ * (width, tiles and staging all 0, the default: small batches, at most 8 RHS
+ * per system and 1024 site-lanes per SM and parity, fewer for the wider
+ * precisions, run the whole solve in one dataflow launch, whose sums are added
+ * in another order; the rest staging 0):
  * 0 links read directly per RHS group; 1 staged in shared memory per work
  * item with asynchronous copies; 2 system-blocked: one block per tile serves
  * every RHS of its system in groups of the RHS-block width, the tile's links

@@ -1,6 +1,7 @@
 // cg.cu — batched conjugate-gradient solver for D D^dag x = b (three to five
 // kernels per iteration, replayed as CUDA-graph chunks, or one persistent
-// launch per solve).
+// launch per solve; small systems without an explicit schedule go to the
+// dataflow kernel of cg_flow.cu).
 //
 // Restates solve_CG_DDdagger (Fermions.cpp:553-617) for the GPU.  D D^dag =
 // m^2 - K^2 and K couples only even and odd sites, so D D^dag is block
@@ -49,13 +50,15 @@
 #include <vector>
 
 #include "cg_common.cuh"
+#include "cg_flow.cuh"
+#include "cg_site.cuh"
 #include "tstage.cuh"
 
 namespace sfh {
 
 namespace {
 
-constexpr int kSums = 4;  // <p,v>, <r,v>, |v|^2, |r|^2
+
 
 // resident 256-thread blocks per SM the hop kernels are compiled for (at most
 // 85 registers a thread for three, 64 for four): up to two lanes a block fit
@@ -153,29 +156,6 @@ __device__ __forceinline__ ItemRange item_range(const CgArgs& a, const CgSys& S,
     r.end = min(first + a.tpi, S.tile0 + (r.q + 1) * S.ntq);
     r.slot = r.q * item_groups(a, S) + j / a.tpi;
     return r;
-}
-
-// neighbour checkerboard indices and hop signs of one output site, computed
-// once and shared by every lane of the block
-struct Nbr {
-    int up[4], dn[4];
-    unsigned eta;  // bit mu: eta_mu(x) = -1
-    bool wu, wd;   // the forward / backward time hop wraps (anti-periodic sign)
-};
-
-__device__ __forceinline__ Nbr neighbours(const Geom& g, const Coord& c)
-{
-    Nbr n;
-    n.eta = 0;
-#pragma unroll
-    for (int mu = 0; mu < 4; ++mu) {
-        n.up[mu] = lex_up(g, c, mu) >> 1;
-        n.dn[mu] = lex_dn(g, c, mu) >> 1;
-        if (eta_sign(c, mu) < 0) n.eta |= 1u << mu;
-    }
-    n.wu = c.x[3] == g.L[3] - 1;
-    n.wd = c.x[3] == 0;
-    return n;
 }
 
 // Link staging: every thread copies the 8 links of its site (4 forward at
@@ -535,39 +515,6 @@ __global__ void __launch_bounds__(kTile) cg_init(CgArgs a)
     }
 }
 
-// FP64 hop of x_hi + x_lo for a lane in a reliable update: thi = K x
-template <int XP, bool COH = false>
-__device__ __forceinline__ void ru_hop1(const CgArgs& a, const CgSys& S, const Coord& c, int q, int i, int rid)
-{
-    const int nq = 1 - q, Vh = S.g.Vh;
-    const void* xhi = rhs_ptr(a, rid, F_XHI);
-    const void* xlo = rhs_ptr(a, rid, F_XLO);
-    Vec3<double> acc;
-    vzero(acc);
-#pragma unroll 1
-    for (int mu = 0; mu < 4; ++mu) {
-        const bool eta_neg = eta_sign(c, mu) < 0;
-        const int lu = lex_up(S.g, c, mu) >> 1, ld = lex_dn(S.g, c, mu) >> 1;
-        const bool wu = (mu == 3) && (c.x[3] == S.g.L[3] - 1);
-        const bool wd = (mu == 3) && (c.x[3] == 0);
-        {
-            Mat3<double> U = GaugeFmt<GP_F64_18>::load(S.U64, q, mu, i, Vh);
-            Vec3<double> x = vaxpy(SpinorFmt<SP_F64>::template load<COH>(xhi, nq, lu, Vh), 1.0,
-                                   vcvt<double>(SpinorFmt<XP>::template load<COH>(xlo, nq, lu, Vh)));
-            vacc(acc, mul_mv(U, x), eta_neg != wu);
-        }
-        {
-            Mat3<double> U = GaugeFmt<GP_F64_18>::load(S.U64, nq, mu, ld, Vh);
-            Vec3<double> x = vaxpy(SpinorFmt<SP_F64>::template load<COH>(xhi, nq, ld, Vh), 1.0,
-                                   vcvt<double>(SpinorFmt<XP>::template load<COH>(xlo, nq, ld, Vh)));
-            vacc(acc, mul_adj_mv(U, x), !(eta_neg != wd));
-        }
-    }
-#pragma unroll
-    for (int k = 0; k < 3; ++k) acc.c[k] = {0.5 * acc.c[k].re, 0.5 * acc.c[k].im};
-    SpinorFmt<SP_F64>::store(rhs_ptr(a, rid, F_THI), q, i, Vh, acc);
-}
-
 // Neighbour staging of one work item's tiles (schedule 6, FP16): buffer
 // k & 1 of [2][NB][W] uint4 words holds tile k's range [i0 - Lt/2,
 // i0 + kTile + Lt/2) of each active lane's input (tstage.cuh), filled by
@@ -756,82 +703,6 @@ __global__ void __launch_bounds__(kTile, (HopOcc<GP, SP, NB, false, RUI>::v))
         }
     } else {
         hop1_item<GP, SP, NB, STG, RUI, NST>(a, items[blockIdx.x], cur);
-    }
-}
-
-// reliable update at the lane's own site: x_hi += x_lo, x_lo = 0,
-// r = b - M x_hi; returns the |r|^2 contribution (FP64)
-template <int SP, int XP, bool COH = false>
-__device__ __forceinline__ double ru_hop2(const CgRhs* a, const CgSys& S, const Coord& c, int q, int i, int rid,
-                                          double m2)
-{
-    typedef typename SpinorFmt<SP>::R RS;
-    const int nq = 1 - q, Vh = S.g.Vh;
-    const void* thi = rhs_ptr(a, rid, F_THI);
-    Vec3<double> acc;
-    vzero(acc);
-#pragma unroll 1
-    for (int mu = 0; mu < 4; ++mu) {
-        const bool eta_neg = eta_sign(c, mu) < 0;
-        const int lu = lex_up(S.g, c, mu) >> 1, ld = lex_dn(S.g, c, mu) >> 1;
-        const bool wu = (mu == 3) && (c.x[3] == S.g.L[3] - 1);
-        const bool wd = (mu == 3) && (c.x[3] == 0);
-        Mat3<double> U = GaugeFmt<GP_F64_18>::load(S.U64, q, mu, i, Vh);
-        vacc(acc, mul_mv(U, SpinorFmt<SP_F64>::template load<COH>(thi, nq, lu, Vh)), eta_neg != wu);
-        Mat3<double> Ud = GaugeFmt<GP_F64_18>::load(S.U64, nq, mu, ld, Vh);
-        vacc(acc, mul_adj_mv(Ud, SpinorFmt<SP_F64>::template load<COH>(thi, nq, ld, Vh)), !(eta_neg != wd));
-    }
-    void* xhi = rhs_ptr(a, rid, F_XHI);
-    void* xlo = rhs_ptr(a, rid, F_XLO);
-    Vec3<double> xn = vaxpy(SpinorFmt<SP_F64>::load_cg(xhi, q, i, Vh), 1.0,
-                            vcvt<double>(SpinorFmt<XP>::load_cg(xlo, q, i, Vh)));
-    SpinorFmt<SP_F64>::store(xhi, q, i, Vh, xn);
-    Vec3<typename SpinorFmt<XP>::R> z;
-    vzero(z);
-    SpinorFmt<XP>::store(xlo, q, i, Vh, z);
-    Vec3<double> b = SpinorFmt<SP_F64>::load(rhs_ptr(a, rid, F_B), q, i, Vh);
-    Vec3<double> res;
-#pragma unroll
-    for (int k = 0; k < 3; ++k) {
-        res.c[k].re = b.c[k].re - (m2 * xn.c[k].re - 0.5 * acc.c[k].re);
-        res.c[k].im = b.c[k].im - (m2 * xn.c[k].im - 0.5 * acc.c[k].im);
-    }
-    // The search direction of the previous update, p = r_iter + beta p_old,
-    // was built from the iterated residual; give it the true one instead,
-    // p = r_true + beta p_old, by adding the correction r_true - r_iter.
-    // Without it the low-precision lanes of ill-conditioned systems lose
-    // their Krylov progress at every update (FP16 storage, eps = 1 links,
-    // m = 0.02 on 16^4: 7648 iterations against FP64's 1564; 1750 with it).
-    void* rp = rhs_ptr(a, rid, F_R);
-    void* pp = rhs_ptr(a, rid, F_P);
-    const Vec3<RS> r_iter = SpinorFmt<SP>::load_cg(rp, q, i, Vh);
-    Vec3<RS> p = SpinorFmt<SP>::load_cg(pp, q, i, Vh);
-#pragma unroll
-    for (int k = 0; k < 3; ++k) {
-        p.c[k].re += (RS)res.c[k].re - r_iter.c[k].re;
-        p.c[k].im += (RS)res.c[k].im - r_iter.c[k].im;
-    }
-    SpinorFmt<SP>::store(pp, q, i, Vh, p);
-    SpinorFmt<SP>::store(rp, q, i, Vh, vcvt<RS>(res));
-    return vdot_re(res, res);
-}
-
-// one site's Re <a, b>: in FP32 for FP32 vectors (exactly the same value in
-// every schedule, added to the FP64 partials), in FP64 for FP64 vectors
-template <typename R>
-__device__ __forceinline__ double site_dot(const Vec3<R>& a, const Vec3<R>& b)
-{
-    if constexpr (sizeof(R) == 4) {
-        float s = a.c[0].re * b.c[0].re;
-        s = fmaf(a.c[0].im, b.c[0].im, s);
-#pragma unroll
-        for (int k = 1; k < 3; ++k) {
-            s = fmaf(a.c[k].re, b.c[k].re, s);
-            s = fmaf(a.c[k].im, b.c[k].im, s);
-        }
-        return (double)s;
-    } else {
-        return vdot_re(a, b);
     }
 }
 
@@ -1759,6 +1630,7 @@ struct CgWorkspace {
     bool timed_out = false;    // the last persistent solve gave up at a barrier
     long long barrier_polls = 0;  // bound on each barrier wait (0: the default)
     int num_sms = 0;
+    int auto_nb = 0;           // RHS-block width without an explicit schedule (0: from the RHS count)
     std::vector<void*> allocs;
     size_t bytes = 0;
     // iteration chunks replayed as one graph launch each
@@ -1776,6 +1648,18 @@ struct CgWorkspace {
         int n;
     };
     std::vector<Items> item_cache;  // work-item lists by RHS-group width
+    // the dataflow kernel's teams (cg_flow.cu), planned at the first use
+    struct Flow {
+        int state = 0;  // 0 not planned, 1 planned, -1 the systems do not suit it
+        FlowPlan plan;
+        size_t words_bytes = 0;
+        FlowTeam* d_teams = nullptr;
+        int* d_blk_team = nullptr;
+        char* d_words = nullptr;  // sums, then the blocks' flags
+        size_t flags_at = 0;
+        char* d_pub = nullptr;    // every RHS's published vectors
+        char** d_pub_ptr = nullptr;
+    } flow;
 
     ~CgWorkspace() { release(); }
     void release_graph()
@@ -1797,6 +1681,7 @@ struct CgWorkspace {
         for (void* p : allocs) cudaFree(p);
         allocs.clear();
         item_cache.clear();
+        flow = Flow();
         d_sys = nullptr; d_rhs = nullptr; d_lanes = nullptr;
         d_tile_sys = nullptr; d_partial = nullptr; d_active = nullptr; d_bar = nullptr; d_rulist = nullptr; d_qctr = nullptr;
     }
@@ -2111,18 +1996,93 @@ static int default_tpi(const CgWorkspace& w, int nb1)
     return items < 4L * std::max(1, w.num_sms) ? 1 : 2;
 }
 
+// the dataflow kernel's plan and buffers, at the first solve that asks; where
+// they do not fit, the per-phase kernels stay
+static cudaError_t flow_buffers(CgWorkspace& w)
+{
+    CgWorkspace::Flow& F = w.flow;
+    FlowPlan& P = F.plan;
+    const int blocks = (int)P.blk_team.size();
+    F.flags_at = P.words * sizeof(uint4);
+    F.words_bytes = F.flags_at + sizeof(unsigned) * blocks;
+    cudaError_t e;
+    if ((e = w.alloc((void**)&F.d_teams, sizeof(FlowTeam) * P.teams.size())) != cudaSuccess) return e;
+    if ((e = w.alloc((void**)&F.d_blk_team, sizeof(int) * blocks)) != cudaSuccess) return e;
+    if ((e = w.alloc((void**)&F.d_words, F.words_bytes)) != cudaSuccess) return e;
+    if ((e = w.alloc((void**)&F.d_pub, P.pub_bytes)) != cudaSuccess) return e;
+    if ((e = w.alloc((void**)&F.d_pub_ptr, sizeof(char*) * P.pub_at.size())) != cudaSuccess) return e;
+    if (!w.d_bar && (e = w.alloc((void**)&w.d_bar, sizeof(GridBar))) != cudaSuccess) return e;
+    std::vector<char*> ptrs;
+    for (size_t at : P.pub_at) ptrs.push_back(F.d_pub + at);
+    if ((e = cudaMemcpy(F.d_teams, P.teams.data(), sizeof(FlowTeam) * P.teams.size(), cudaMemcpyHostToDevice)) !=
+        cudaSuccess)
+        return e;
+    if ((e = cudaMemcpy(F.d_blk_team, P.blk_team.data(), sizeof(int) * blocks, cudaMemcpyHostToDevice)) != cudaSuccess)
+        return e;
+    return cudaMemcpy(F.d_pub_ptr, ptrs.data(), sizeof(char*) * ptrs.size(), cudaMemcpyHostToDevice);
+}
+
+static cudaError_t flow_prepare(CgWorkspace& w)
+{
+    w.flow.state = -1;
+    if (!flow_plan(w.sys, w.prec, w.num_sms, &w.flow.plan)) return cudaSuccess;
+    const cudaError_t e = flow_buffers(w);
+    if (e == cudaSuccess) w.flow.state = 1;
+    if (e != cudaErrorMemoryAllocation) return e;
+    cudaGetLastError();
+    return cudaSuccess;
+}
+
+// the whole solve (after cg_init) in one dataflow launch
+static cudaError_t flow_solve(CgWorkspace& w, const CgArgs& a, cudaStream_t stream)
+{
+    const CgWorkspace::Flow& F = w.flow;
+    cudaError_t e;
+    // no word of an earlier solve carries a tag this one waits for
+    if ((e = cudaMemsetAsync(F.d_words, 0, F.words_bytes, stream)) != cudaSuccess) return e;
+    if ((e = cudaMemsetAsync(F.d_pub, 0, F.plan.pub_bytes, stream)) != cudaSuccess) return e;
+    if ((e = cudaMemsetAsync(&w.d_bar->err, 0, sizeof(int), stream)) != cudaSuccess) return e;
+    FlowArgs f;
+    f.teams = F.d_teams;
+    f.blk_team = F.d_blk_team;
+    f.sums = (uint4*)F.d_words;
+    f.flags = (unsigned*)(F.d_words + F.flags_at);
+    f.pub = F.d_pub_ptr;
+    f.err = &w.d_bar->err;
+    f.polls = kFlowPolls;  // about 0.6 us each
+    if ((e = flow_launch(w.prec, a, f, F.plan, stream)) != cudaSuccess) return e;
+    w.launches += 1;
+    int err = 0;
+    if ((e = cudaMemcpyAsync(&err, &w.d_bar->err, sizeof(int), cudaMemcpyDeviceToHost, stream)) != cudaSuccess) return e;
+    if ((e = finish_solve(w, stream)) != cudaSuccess) return e;
+    w.timed_out = err != 0;
+    return cudaSuccess;
+}
+
 // Solve every lane of a built workspace.  nb1 / nb2: RHS-block widths of the
 // two hop kernels (0 = from the largest RHS count); tpi: tiles per block of
 // the iteration kernels (0 = default_tpi); stage: hop kernels stage their
-// links in shared memory (reduced precisions only).  Returns a cudaError.
+// links in shared memory (reduced precisions only); prefer_flow: the dataflow
+// kernel where the systems suit it, whatever the schedule.  Returns a cudaError.
 static cudaError_t workspace_solve(CgWorkspace& w, double tol, int maxit, double delta, int nb1, int nb2,
-                                   int tpi, int stage, cudaStream_t stream, PhaseTimes* timing = nullptr)
+                                   int tpi, int stage, cudaStream_t stream, PhaseTimes* timing = nullptr,
+                                   bool prefer_flow = false)
 {
     int max_nrhs = 1;
     for (const CgSys& S : w.sys) max_nrhs = std::max(max_nrhs, S.nrhs);
     const bool f64 = w.prec == SFH_PREC_F64;
-    if (nb1 <= 0) nb1 = default_nb(max_nrhs, f64 ? 2 : 8);
-    if (nb2 <= 0) nb2 = default_nb(max_nrhs, f64 ? 2 : 4);
+    // without an explicit schedule, systems that fit the SMs' shared memory
+    // take the dataflow kernel (flow_plan says where the line lies)
+    bool flow = false;
+    if (!timing && (prefer_flow || (nb1 <= 0 && nb2 <= 0 && tpi <= 0 && stage == 0))) {
+        if (w.flow.state == 0) {
+            const cudaError_t fe = flow_prepare(w);
+            if (fe != cudaSuccess) return fe;
+        }
+        flow = w.flow.state > 0;
+    }
+    if (nb1 <= 0) nb1 = w.auto_nb > 0 ? w.auto_nb : default_nb(max_nrhs, f64 ? 2 : 8);
+    if (nb2 <= 0) nb2 = w.auto_nb > 0 ? w.auto_nb : default_nb(max_nrhs, f64 ? 2 : 4);
     w.nb = nb1;
     for (CgLane& L : w.lanes_h) {
         L.mode[0] = L.mode[1] = LM_ACTIVE;
@@ -2188,6 +2148,12 @@ static cudaError_t workspace_solve(CgWorkspace& w, double tol, int maxit, double
     w.launches = 1;
     w.timed_out = false;
     if ((e = cudaGetLastError()) != cudaSuccess) return e;
+    if (flow) {
+        e = flow_solve(w, a, stream);
+        if (e != cudaErrorCooperativeLaunchTooLarge) return e;
+        cudaGetLastError();  // fewer SMs than the device reports: the per-phase kernels
+        w.flow.state = -1;
+    }
     if (k.pers) return persistent_solve(w, k, a, stream, timing);
     if (!timing && (e = ensure_graph(w, k, a, tol, maxit, delta)) != cudaSuccess) return e;
     // timed solves: the same kernels and work items, launched one by one
@@ -2300,6 +2266,7 @@ struct sfh_batch {
     cudaStream_t stream = nullptr;
     bool own_stream = false;
     int prec = 0, flags = 0, nb = 0, nb2 = 0, tpi = 0, stage_links = 0;
+    bool tuned_flow = false;  // the autotuner found the dataflow kernel faster than its schedule
     double delta = 0.1;  // reliable-update threshold of the mixed precisions (set at creation)
     std::vector<sfh_system_desc> desc;
     std::vector<sfh::Geom> geoms;
@@ -2454,6 +2421,7 @@ extern "C" int sfh_batch_set_rhs_block(sfh_batch* b, int width)
     if (!b || width < 0 || width > 8) return SFH_ERR_INVALID;
     b->nb = width;
     b->nb2 = width;
+    b->tuned_flow = false;
     return SFH_OK;
 }
 
@@ -2462,6 +2430,7 @@ extern "C" int sfh_batch_set_hop_widths(sfh_batch* b, int hop1_width, int hop2_w
     if (!b || hop1_width < 0 || hop1_width > 8 || hop2_width < 0 || hop2_width > 8) return SFH_ERR_INVALID;
     b->nb = hop1_width;
     b->nb2 = hop2_width;
+    b->tuned_flow = false;
     return SFH_OK;
 }
 
@@ -2496,8 +2465,8 @@ extern "C" int sfh_batch_solve(sfh_batch* b, double tol, int maxit)
 {
     if (!b || !(tol > 0.0) || maxit <= 0) return SFH_ERR_INVALID;
     cudaSetDevice(b->device);
-    int st = batch_cuda(b, sfh::workspace_solve(b->ws, tol, maxit, b->delta, b->nb, b->nb2, b->tpi, b->stage_links, b->stream),
-                        "batched CG");
+    int st = batch_cuda(b, sfh::workspace_solve(b->ws, tol, maxit, b->delta, b->nb, b->nb2, b->tpi, b->stage_links, b->stream,
+                                                nullptr, b->tuned_flow), "batched CG");
     if (st) return st;
     if (b->ws.timed_out)
         return batch_err(b, SFH_ERR_TIMEOUT, "batched CG: a bounded device wait (grid barrier or neighbour staging) gave up");
@@ -2704,7 +2673,8 @@ int ctx_solve_pair_device(sfh_ctx* c, const void* const b_eo[2], void* const x_e
     // hops slower than a one-RHS item (24^4, FP32 storage: 62.2 ms for the
     // pair at width 1 against 74.4 ms at width 2 and 64.5 ms for two solves)
     const bool lowp = prec != SFH_PREC_F64;
-    const int nb = lowp ? (c->sched_nb > 0 ? c->sched_nb : 1) : 0;
+    w->auto_nb = lowp ? 1 : 0;
+    const int nb = lowp ? c->sched_nb : 0;
     e = workspace_solve(*w, tol, maxit, default_reliable_delta(prec), nb, nb, lowp ? c->sched_tpi : 0,
                         lowp ? c->sched_stage : 0, c->stream);
     if (e != cudaSuccess) return cuda_check(c, e, "cg pair solve");
@@ -2844,8 +2814,8 @@ extern "C" int sfh_batch_kernel_launches(sfh_batch* b, long* n)
 
 // Autotuner: times a capped solve (probe_iters iterations, no lane converges)
 // for every RHS-block width, tiles-per-block count and link staging mode
-// (read directly, staged per work item, system-blocked) and keeps the
-// fastest.
+// (read directly, staged per work item, system-blocked), and the dataflow
+// kernel, and keeps the fastest.
 extern "C" int sfh_batch_autotune(sfh_batch* b, int probe_iters, int* best_width)
 {
     if (!b || probe_iters < 1) return SFH_ERR_INVALID;
@@ -2884,6 +2854,16 @@ extern "C" int sfh_batch_autotune(sfh_batch* b, int probe_iters, int* best_width
                     bs = stage;
                 }
             }
+    // the dataflow kernel against the fastest schedule, which stays the batch's
+    double flow = 1e300;
+    for (int rep = 0; rep < 2 && b->ws.flow.state >= 0; ++rep) {
+        auto t0 = std::chrono::steady_clock::now();
+        cudaError_t e = sfh::workspace_solve(b->ws, 1e-30, probe_iters, 0.1, bw, bw2, bt, bs, b->stream, nullptr, true);
+        if (e != cudaSuccess) return batch_cuda(b, e, "autotune");
+        if (b->ws.flow.state > 0)
+            flow = std::chrono::duration<double>(std::chrono::steady_clock::now() - t0).count();
+    }
+    b->tuned_flow = flow < best;
     b->nb = bw;
     b->nb2 = bw2;
     b->tpi = bt;
@@ -2899,6 +2879,7 @@ extern "C" int sfh_batch_set_schedule(sfh_batch* b, int width, int tiles_per_blo
     b->tpi = tiles_per_block;
     if (stage_links < 0 || stage_links > 7) return SFH_ERR_INVALID;
     b->stage_links = stage_links;
+    b->tuned_flow = false;
     return SFH_OK;
 }
 

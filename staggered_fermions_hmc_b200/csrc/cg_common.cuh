@@ -16,6 +16,7 @@ namespace sfh {
 // (p = r), used after the FP64 residual update of restarting lanes
 enum { LM_ACTIVE = 0, LM_RU = 1, LM_DONE = 2, LM_FAILED = 3, LM_LAST = 4, LM_RESTART = 5 };
 constexpr int kTile = 256;
+constexpr int kSums = 4;  // <p,v>, <r,v>, |v|^2, |r|^2
 
 struct CgSys {
     Geom g;

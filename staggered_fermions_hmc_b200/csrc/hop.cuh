@@ -185,30 +185,40 @@ __device__ __forceinline__ void acc_f32x2(Cx<float>& acc, unsigned long long f2,
     asm("mov.b64 {%0, %1}, %2;" : "=f"(acc.re), "=f"(acc.im) : "l"(d));
 }
 
-// acc += f (U v) (ADJ false) or acc += f (U^dag v) (ADJ true) for the
-// stored FP16 vector word w (three half2 pairs and the site scale sc):
-// f = s sc, products in half2
+// y = U v (ADJ false) or U^dag v (ADJ true) for the three half2 pairs of a
+// stored FP16 vector word, in half2
 template <bool ADJ>
-__device__ __forceinline__ void hop_half_word(Vec3<float>& acc, const __half2 (&U)[9], const uint4 w, float f)
+__device__ __forceinline__ void half_products(const __half2 (&U)[9], const uint4 w, __half2 (&y)[3])
 {
     const __half2 v[3] = {h2_bits(w.x), h2_bits(w.y), h2_bits(w.z)};
-    const unsigned long long f2 = f32x2_bcast(f * __uint_as_float(w.w));
     __half2 vp[3];
 #pragma unroll
     for (int k = 0; k < 3; ++k) vp[k] = ADJ ? __hneg2(h2_perp(v[k])) : h2_perp(v[k]);
 #pragma unroll
     for (int r = 0; r < 3; ++r) {
         // row r of U (U_rk) or column r (conj(U_kr)); conj(u) v = u.re v - u.im v_perp
-        __half2 y = __hmul2(__low2half2(U[ADJ ? r : 3 * r]), v[0]);
-        y = __hfma2(__high2half2(U[ADJ ? r : 3 * r]), vp[0], y);
+        y[r] = __hmul2(__low2half2(U[ADJ ? r : 3 * r]), v[0]);
+        y[r] = __hfma2(__high2half2(U[ADJ ? r : 3 * r]), vp[0], y[r]);
 #pragma unroll
         for (int k = 1; k < 3; ++k) {
             const __half2 u = U[ADJ ? 3 * k + r : 3 * r + k];
-            y = __hfma2(__low2half2(u), v[k], y);
-            y = __hfma2(__high2half2(u), vp[k], y);
+            y[r] = __hfma2(__low2half2(u), v[k], y[r]);
+            y[r] = __hfma2(__high2half2(u), vp[k], y[r]);
         }
-        acc_f32x2(acc.c[r], f2, __half22float2(y));
     }
+}
+
+// acc += f (U v) (ADJ false) or acc += f (U^dag v) (ADJ true) for the
+// stored FP16 vector word w (three half2 pairs and the site scale sc):
+// f = s sc, products in half2
+template <bool ADJ>
+__device__ __forceinline__ void hop_half_word(Vec3<float>& acc, const __half2 (&U)[9], const uint4 w, float f)
+{
+    const unsigned long long f2 = f32x2_bcast(f * __uint_as_float(w.w));
+    __half2 y[3];
+    half_products<ADJ>(U, w, y);
+#pragma unroll
+    for (int r = 0; r < 3; ++r) acc_f32x2(acc.c[r], f2, __half22float2(y[r]));
 }
 
 // hop_half_word for the vector of site j of parity nq in global memory

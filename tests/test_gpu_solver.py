@@ -563,3 +563,79 @@ def test_batch_rhs_at_their_own_masses(sfh, orc, precision):
         assert iters[0] > iters[1] > iters[2]  # lighter masses need more iterations
     finally:
         B.close()
+
+
+def _solve_default_and_per_phase(sfh, orc, systems, precision, full_lattice=False, max_iter=20000):
+    """Solutions of a batch without a schedule (the dataflow kernel for these
+    sizes) and with the per-phase kernels' schedule, and the inputs."""
+    fields = [(orc.random_gauge(d, 0.4 + 0.6 * (k % 2), 1500 + k), [orc.random_spinor(d, 1600 + 10 * k + j) for j in range(n)])
+              for k, (d, m, n) in enumerate(systems)]
+    out = []
+    for schedule in ((0, 0, 0), (1, 1, 0)):
+        B = sfh.Batch(systems, precision=precision, full_lattice=full_lattice)
+        B.set_schedule(*schedule)
+        for k, (U, bs) in enumerate(fields):
+            B.set_gauge(k, U)
+            for j, b in enumerate(bs):
+                B.set_rhs(k, j, b)
+        B.solve(tol=1e-10, max_iter=max_iter)
+        if schedule == (0, 0, 0):
+            assert B.kernel_launches() == 2  # cg_init and the dataflow kernel
+            first = [B.solution(k, j) for k, (d, m, n) in enumerate(systems) for j in range(n)]
+            B.solve(tol=1e-10, max_iter=max_iter)  # its words carry the last solve's tags
+            again = [B.solution(k, j) for k, (d, m, n) in enumerate(systems) for j in range(n)]
+            assert all(np.array_equal(a, b) for a, b in zip(first, again))
+        out.append(([B.solution(k, j) for k, (d, m, n) in enumerate(systems) for j in range(n)],
+                    [B.info(k, j) for k, (d, m, n) in enumerate(systems) for j in range(n)]))
+        B.close()
+    return fields, out
+
+
+@pytest.mark.parametrize("precision", ["f64", "f32", "f16", "bf16", "f32_18"])
+@pytest.mark.parametrize("systems", [
+    [((4, 4, 4, 4), 0.1, 1)],                                              # a few blocks of one round
+    [((2, 4, 6, 2), 0.2, 2)],                                              # fewer sites than a block's least share
+    [((6, 10, 6, 10), 0.1, 1)],                                            # the last block's share is partial
+    [((8, 8, 8, 8), 0.05, 3), ((4, 6, 8, 10), 0.1, 8), ((2, 2, 2, 4), 0.2, 1)],  # teams of unequal size, 8 RHS
+    [((12, 12, 12, 24), 0.2, 1)],                                          # several rounds or threads per site = 1
+])
+def test_dataflow_solve_matches_per_phase_kernels(sfh, orc, systems, precision):
+    """The dataflow kernel's solutions against the per-phase kernels' (the
+    iteration counts may differ by the rounding of the sums) and against the
+    oracle's operator: true residual below 1.5 tol, difference below
+    cond(M) 2 tol with cond(M) <= (m^2 + 16) / m^2."""
+    tol = 1e-10
+    fields, (flow, phase) = _solve_default_and_per_phase(sfh, orc, systems, precision)
+    at = 0
+    for (dims, mass, nrhs), (U, bs) in zip(systems, fields):
+        for b in bs:
+            X, Xp = flow[0][at], phase[0][at]
+            assert flow[1][at]["status"] == 0
+            assert abs(flow[1][at]["iters"] - phase[1][at]["iters"]) <= 2 + phase[1][at]["iters"] // 50
+            assert true_resid(orc, dims, mass, U, b, X) < 1.5 * tol
+            assert np.linalg.norm(X - Xp) <= 2 * tol * (mass ** 2 + 16) / mass ** 2 * np.linalg.norm(Xp)
+            at += 1
+
+
+def test_dataflow_solve_full_lattice_masses_and_stops(sfh, orc):
+    """The dataflow kernel with both parities in one lane, several masses on
+    the same links, a zero right-hand side (X = 0) and an iteration limit
+    (SFH_ERR_NOCONV)."""
+    dims, tol = (6, 4, 8, 6), 1e-10
+    U = orc.random_gauge(dims, 0.7, 1700)
+    bs = [orc.random_spinor(dims, 1701), np.zeros(6 * 1152), orc.random_spinor(dims, 1702)]
+    for precision, full in (("f64", True), ("f64", False), ("f32", False)):
+        B = sfh.Batch([(dims, 0.1, 3)], precision=precision, full_lattice=full)
+        B.set_gauge(0, U)
+        for j, b in enumerate(bs):
+            B.set_rhs(0, j, b)
+        B.set_rhs_mass(0, 2, 0.4)
+        B.solve(tol=tol)
+        assert B.kernel_launches() == 2
+        assert true_resid(orc, dims, 0.1, U, bs[0], B.solution(0, 0)) < 1.5 * tol
+        assert np.all(B.solution(0, 1) == 0)
+        assert true_resid(orc, dims, 0.4, U, bs[2], B.solution(0, 2)) < 1.5 * tol
+        with pytest.raises(sfh.SfhError) as e:
+            B.solve(tol=tol, max_iter=5)
+        assert e.value.status == sfh.SFH_ERR_NOCONV
+        B.close()
