@@ -2,16 +2,28 @@
 // force, momentum kick, link update U <- exp(i eps P) U, and the FP64
 // reductions Tr P^2, gauge action, plaquette and Re<phi, X>.
 //
-// Fields are FP64 in the even-odd SoA layout of sfh_core.cuh.  One thread per
-// link (parity p, direction mu, checkerboard site i).  Staples are products of
-// links along lattice paths (periodic in every direction for gauge links,
-// Lattice.cpp:213-235); the paths are those of compute_staple_sum_at_link
-// (Lattice.cpp:249-313) and compute_rectangle_staple_sum_at_link
-// (Lattice.cpp:315-499), each written as the walk from x+mu back to x so that
-// U_mu(x) * staple is a closed loop.
+// Fields are FP64 in the even-odd SoA layout of sfh_core.cuh, links indexed by
+// (parity p, direction mu, checkerboard site i).  Gauge links are periodic in
+// every direction (Lattice.cpp:213-235); the staple paths are those of
+// compute_staple_sum_at_link (Lattice.cpp:249-313) and
+// compute_rectangle_staple_sum_at_link (Lattice.cpp:315-499).
+//
+// Staples: the paths of one link through one direction +-nu share their
+// pieces, so that the plaquette staple and the three rectangles of that side
+// take 11 products of 3x3 matrices (staple_side) instead of the 18 of walking
+// each path on its own; a block of six warps gives each of the six sides of 32
+// links to one warp (the directions are then uniform in a warp, a thread holds
+// four matrices instead of six, and the sides' links meet in the L1), and adds
+// the sides through shared memory.  The products are FMA chains (su3.cuh).
+// Measured on the B200, one thread and whole walks per link -> this: gauge
+// force 363 -> 250 us at 16^4, 2196 -> 1399 us at 24^4; staples 2470 -> 1415 us;
+// a heatbath sweep 3.57 -> 0.91 ms at 16^4, 18.1 -> 4.1 ms at 24^4.  It runs at
+// 14 TFLOP/s, 0.4 of the FP64 pipe, latency bound on 12 warps per SM (168
+// registers): a third of the stalls are link loads, a fifth each FMA latency
+// and instruction fetch.  A row of the staples per thread (80 registers, 24
+// warps, every link read by three threads) was bound by the L1: 2696 us.
 #include "sfh_internal.h"
 #include "su3.cuh"
-#include "walk.cuh"
 
 namespace sfh {
 
@@ -19,58 +31,214 @@ namespace {
 
 constexpr int kThreads = 128;
 
-// product of links along a path; step s > 0 walks +(s-1), s < 0 walks -(-s-1)
-template <int N>
-__device__ __forceinline__ M3 path(const void* U, const Geom& g, Walker w, const int (&steps)[N])
+__device__ __forceinline__ int coord_of(const Coord& c, int mu)
 {
-    M3 m = m3_id();
+    return mu == 0 ? c.x[0] : (mu == 1 ? c.x[1] : (mu == 2 ? c.x[2] : c.x[3]));
+}
+
+__device__ __forceinline__ int extent_of(const Geom& g, int mu)
+{
+    return mu == 0 ? g.L[0] : (mu == 1 ? g.L[1] : (mu == 2 ? g.L[2] : g.L[3]));
+}
+
+// offset of x + k mu, |k| <= 2 <= L
+__device__ __forceinline__ int step_offset(const Geom& g, const Coord& c, int mu, int k)
+{
+    const int L = extent_of(g, mu), x = coord_of(c, mu);
+    int y = x + k;
+    if (y < 0) y += L;
+    if (y >= L) y -= L;
+    return (y - x) * lex_stride(g, mu);
+}
+
+// The links around a site x on one side, +nu or -nu, of direction mu:
+// M(m, k) = U_mu(x + m mu + k side) and D(m, k), the step from x + m mu +
+// k side further along the side: U_nu there, or U_nu^dag of the site below.
+// One code for both sides (a D's elements are read transposed and their
+// imaginary parts' signs flipped), at the same speed as a copy for each.
+struct Side {
+    const double2 *Um, *Un;   // the links of mu and of nu at x's parity ...
+    const double2 *Vm, *Vn;   // ... and at the other one
+    int Vh, lex;
+    int m[4];                 // offsets of x + (k - 1) mu
+    int sm[3], sd[2];         // of x + k side, and of where its D starts
+    int rs, cs;               // a D's row and column strides
+    unsigned conj;            // its imaginary parts' sign flip
+    bool up;
+};
+
+__device__ __forceinline__ Side make_side(const void* U, const Geom& g, const Coord& c, int p, int mu, int nu, bool up)
+{
+    Side s;
+    auto field = [&](int par, int a) { return (const double2*)U + ((size_t)(par * 4 + a) * 9) * g.Vh; };
+    s.Um = field(p, mu);
+    s.Vm = field(1 - p, mu);
+    s.Un = field(up ? p : 1 - p, nu);
+    s.Vn = field(up ? 1 - p : p, nu);
+    s.Vh = g.Vh;
+    s.lex = c.lex;
+    s.up = up;
 #pragma unroll
-    for (int k = 0; k < N; ++k) {
-        int s = steps[k];
-        int mu = (s > 0 ? s : -s) - 1;
-        if (s > 0) {
-            m = m3_mul(m, link_at(U, g, w, mu));
-            walk(g, w, mu, +1);
-        } else {
-            walk(g, w, mu, -1);
-            m = m3_mul_adj(m, link_at(U, g, w, mu));
+    for (int k = 0; k < 4; ++k) s.m[k] = step_offset(g, c, mu, k - 1);
+#pragma unroll
+    for (int k = 0; k < 3; ++k) s.sm[k] = step_offset(g, c, nu, up ? k : -k);
+    s.sd[0] = up ? s.sm[0] : s.sm[1];
+    s.sd[1] = up ? s.sm[1] : s.sm[2];
+    s.rs = up ? 3 * g.Vh : g.Vh;
+    s.cs = up ? g.Vh : 3 * g.Vh;
+    s.conj = up ? 0u : 0x80000000u;
+    return s;
+}
+
+template <int M, int K>
+__device__ __forceinline__ M3 side_m(const Side& s)
+{
+    const double2* b = (((M + K) & 1) ? s.Vm : s.Um) + ((s.lex + s.m[M + 1] + s.sm[K]) >> 1);
+    M3 o;
+#pragma unroll
+    for (int k = 0; k < 9; ++k) {
+        const double2 v = __ldg(b + (size_t)k * s.Vh);
+        o.e[k] = {v.x, v.y};
+    }
+    return o;
+}
+
+template <int M, int K>
+__device__ __forceinline__ M3 side_d(const Side& s)
+{
+    const double2* b = (((M + K) & 1) ? s.Vn : s.Un) + ((s.lex + s.m[M + 1] + s.sd[K]) >> 1);
+    M3 o;
+#pragma unroll
+    for (int i = 0; i < 3; ++i)
+#pragma unroll
+        for (int j = 0; j < 3; ++j) {
+            const double2 v = __ldg(b + i * s.rs + j * s.cs);
+            o.e[3 * i + j] = {v.x, __hiloint2double(__double2hiint(v.y) ^ (int)s.conj, __double2loint(v.y))};
         }
+    return o;
+}
+
+// The staples of U_mu(x) on one side, as walks from x to x + mu:
+//   T  = D0 M1 D2^dag                      D0 = D(0,0), M1 = M(0,1), D2 = D(1,0)
+//   R1 = D0 [D M D^dag](one step out) D2^dag
+//   R2 = [M^dag D M](x - mu) M1 D2^dag      (starts backwards)
+//   R3 = D0 M1 [M D^dag M^dag](x + mu)      (overshoots)
+// SPLIT: S = T, R = R1 + R2 + R3; else S = c1 T + c2 (R1 + R2 + R3).
+template <bool SPLIT>
+__device__ __forceinline__ void staple_side(const Side& s, double c1, double c2, M3& S, M3& R)
+{
+    M3 A, B, t;
+    t = m3_mul(side_d<0, 1>(s), side_m<0, 2>(s));
+    A = m3_mul_adj(t, side_d<1, 1>(s));
+    B = m3_mul(side_d<0, 0>(s), A);                       // R1 without its last step
+    t = m3_adj_mul(side_m<-1, 0>(s), side_d<-1, 0>(s));
+    A = m3_mul(t, side_m<-1, 1>(s));
+    {
+        const M3 M1 = side_m<0, 1>(s);
+        m3_mul_to<true>(B, A, M1);                        // + R2's
+        A = m3_mul(side_d<0, 0>(s), M1);
+    }
+    if constexpr (SPLIT) {
+        const M3 D2 = side_d<1, 0>(s);
+        S = m3_mul_adj(A, D2);
+        R = m3_mul_adj(B, D2);
+    } else {
+#pragma unroll
+        for (int k = 0; k < 9; ++k) B.e[k] = {fma(c2, B.e[k].re, c1 * A.e[k].re), fma(c2, B.e[k].im, c1 * A.e[k].im)};
+        S = m3_mul_adj(B, side_d<1, 0>(s));
+    }
+    t = m3_mul_adj(side_m<1, 1>(s), side_d<2, 0>(s));
+    B = m3_mul_adj(t, side_m<1, 0>(s));
+    if constexpr (SPLIT) {
+        m3_mul_to<true>(R, A, B);
+    } else {
+#pragma unroll
+        for (int k = 0; k < 9; ++k) A.e[k] = {c2 * A.e[k].re, c2 * A.e[k].im};
+        m3_mul_to<true>(S, A, B);
+    }
+}
+
+// the links of x's plane mu, nu for the loops that start there
+struct PlaneSite {
+    const double2* U;
+    int Vh, lex, p;
+    int m[3], n[3];  // offsets of x + k mu and of x + k nu
+};
+
+__device__ __forceinline__ PlaneSite plane_site(const void* U, const Geom& g, const Coord& c, int p, int mu, int nu)
+{
+    PlaneSite s;
+    s.U = (const double2*)U;
+    s.Vh = g.Vh;
+    s.lex = c.lex;
+    s.p = p;
+#pragma unroll
+    for (int k = 0; k < 3; ++k) {
+        s.m[k] = step_offset(g, c, mu, k);
+        s.n[k] = step_offset(g, c, nu, k);
+    }
+    return s;
+}
+
+// U_a(x + dm mu + dn nu)
+__device__ __forceinline__ M3 plane_link(const PlaneSite& s, int a, int dm, int dn)
+{
+    const int i = (s.lex + s.m[dm] + s.n[dn]) >> 1, par = (s.p + dm + dn) & 1;
+    const double2* b = s.U + ((size_t)(par * 4 + a) * 9) * s.Vh + i;
+    M3 m;
+#pragma unroll
+    for (int k = 0; k < 9; ++k) {
+        const double2 v = __ldg(b + (size_t)k * s.Vh);
+        m.e[k] = {v.x, v.y};
     }
     return m;
 }
 
-// A1 (plaquette staples) and A2 (rectangle staples) of link (x, mu); RECT
-// false: A1 alone (the same paths in the same order, A2 left zero)
-template <bool RECT = true>
-__device__ void staples(const void* U, const Geom& g, const Walker& x, int mu, M3& A1, M3& A2)
+// Blocks of the staple kernels: six warps, one side of 32 links each.
+constexpr int kSides = 6, kSideThreads = 32 * kSides;
+
+// the sides' staples of the block's 32 links: 18 doubles each
+struct SideSum {
+    double e[kSides][18][32];
+};
+
+// the staples of this thread's link on its warp's side (staple_side)
+template <bool SPLIT = false>
+__device__ __forceinline__ void side_staples(const void* U, const Geom& g, const Coord& c, int p, int mu, double c1,
+                                             double c2, M3& S, M3& R)
 {
-    Walker xp = x;
-    walk(g, xp, mu, +1);
-    const int M = mu + 1;
-    A1 = m3_zero();
-    A2 = m3_zero();
-#pragma unroll 1
-    for (int nu = 0; nu < 4; ++nu) {
-        if (nu == mu) continue;
-        const int N = nu + 1;
-        const int top[3] = {+N, -M, -N};
-        const int bot[3] = {-N, -M, +N};
-        m3_acc(A1, path(U, g, xp, top));
-        m3_acc(A1, path(U, g, xp, bot));
-        if constexpr (!RECT) continue;
-        const int r1[5] = {-N, -N, -M, +N, +N};
-        const int r2[5] = {+N, +N, -M, -N, -N};
-        const int r3[5] = {+M, -N, -M, -M, +N};
-        const int r4[5] = {+N, -M, -M, -N, +M};
-        const int r5[5] = {-N, -M, -M, +N, +M};
-        const int r6[5] = {+M, +N, -M, -M, -N};
-        m3_acc(A2, path(U, g, xp, r1));
-        m3_acc(A2, path(U, g, xp, r2));
-        m3_acc(A2, path(U, g, xp, r3));
-        m3_acc(A2, path(U, g, xp, r4));
-        m3_acc(A2, path(U, g, xp, r5));
-        m3_acc(A2, path(U, g, xp, r6));
+    const int side = threadIdx.x >> 5, k = side >> 1;
+    staple_side<SPLIT>(make_side(U, g, c, p, mu, k + (k >= mu ? 1 : 0), !(side & 1)), c1, c2, S, R);
+}
+
+// adds the six sides (into e[0]); ends with the block synchronised
+__device__ __forceinline__ void sum_sides(SideSum& sum, const M3& S)
+{
+    const int side = threadIdx.x >> 5, lane = threadIdx.x & 31;
+#pragma unroll
+    for (int k = 0; k < 9; ++k) {
+        sum.e[side][2 * k][lane] = S.e[k].re;
+        sum.e[side][2 * k + 1][lane] = S.e[k].im;
     }
+    __syncthreads();
+#pragma unroll
+    for (int e = 0; e < 3; ++e) {
+        const int k = 3 * side + e;
+        double x = sum.e[0][k][lane];
+#pragma unroll
+        for (int w = 1; w < kSides; ++w) x += sum.e[w][k][lane];
+        sum.e[0][k][lane] = x;
+    }
+    __syncthreads();
+}
+
+__device__ __forceinline__ M3 side_sum(const SideSum& sum)
+{
+    const int lane = threadIdx.x & 31;
+    M3 S;
+#pragma unroll
+    for (int k = 0; k < 9; ++k) S.e[k] = {sum.e[0][2 * k][lane], sum.e[0][2 * k + 1][lane]};
+    return S;
 }
 
 // F = -i f (Q - Q^dag), trace removed
@@ -88,29 +256,13 @@ __device__ __forceinline__ M3 antiherm_force(const M3& Q, double f)
     return F;
 }
 
-// Fermions.cpp:372-384: F_g = -i (beta/12) (U V - (U V)^dag), V = c11 A1 + c12 A2
-__device__ __forceinline__ M3 gauge_force_link(const void* U, const Geom& g, const Walker& x, int mu, double beta,
-                                               double c11, double c12)
+__device__ __forceinline__ Vec3<double> spinor_at(const void* f, int par, int i, int Vh)
 {
-    M3 A1, A2;
-    staples(U, g, x, mu, A1, A2);
-    M3 Vs;
-#pragma unroll
-    for (int k = 0; k < 9; ++k)
-        Vs.e[k] = {c11 * A1.e[k].re + c12 * A2.e[k].re, c11 * A1.e[k].im + c12 * A2.e[k].im};
-    M3 Q = m3_mul(link_at(U, g, x, mu), Vs);
-    return antiherm_force(Q, beta / 12.0);
-}
-
-__device__ __forceinline__ Vec3<double> spinor_at(const void* f, const Geom& g, const Walker& w)
-{
-    int par = (w.x[0] + w.x[1] + w.x[2] + w.x[3]) & 1;
-    int i = lex_of(g, w) >> 1;
-    const double2* b = (const double2*)f + (size_t)par * 3 * g.Vh + i;
+    const double2* b = (const double2*)f + (size_t)par * 3 * Vh + i;
     Vec3<double> v;
 #pragma unroll
     for (int c = 0; c < 3; ++c) {
-        double2 t = __ldg(b + (size_t)c * g.Vh);
+        double2 t = __ldg(b + (size_t)c * Vh);
         v.c[c] = {t.x, t.y};
     }
     return v;
@@ -119,16 +271,13 @@ __device__ __forceinline__ Vec3<double> spinor_at(const void* f, const Geom& g, 
 // Fermions.cpp:443-515: c = eta bc / 4, A_f = (U Y(x+mu)) X(x)^dag,
 // A_b = Y(x) X(x+mu)^dag U^dag, F = -i c [(A_f - A_f^dag) + (A_b - A_b^dag)]
 __device__ __forceinline__ M3 fermion_force_link(const void* U, const void* X, const void* Y, const Geom& g,
-                                                 const Walker& x, int mu)
+                                                 const Coord& x, int p, int mu)
 {
-    Walker xu = x;
-    walk(g, xu, mu, +1);
-    int eta = 0;
-    for (int nu = 0; nu < mu; ++nu) eta += x.x[nu];
-    double c = 0.25 * ((eta & 1) ? -1.0 : 1.0) * ((mu == 3 && x.x[3] == g.L[3] - 1) ? -1.0 : 1.0);
-    M3 Ux = link_at(U, g, x, mu);
-    Vec3<double> Xx = spinor_at(X, g, x), Xu = spinor_at(X, g, xu);
-    Vec3<double> Yx = spinor_at(Y, g, x), Yu = spinor_at(Y, g, xu);
+    const int i = x.lex >> 1, j = (x.lex + step_offset(g, x, mu, 1)) >> 1;
+    const double c = 0.25 * eta_sign(x, mu) * ((mu == 3 && x.x[3] == g.L[3] - 1) ? -1.0 : 1.0);
+    M3 Ux = ld_link(U, p, mu, i, g.Vh);
+    Vec3<double> Xx = spinor_at(X, p, i, g.Vh), Xu = spinor_at(X, 1 - p, j, g.Vh);
+    Vec3<double> Yx = spinor_at(Y, p, i, g.Vh), Yu = spinor_at(Y, 1 - p, j, g.Vh);
     Vec3<double> uy = mul_mv(Ux, Yu);
     M3 Af, T;
 #pragma unroll
@@ -153,19 +302,10 @@ __device__ __forceinline__ M3 fermion_force_link(const void* U, const void* X, c
     return F;
 }
 
-// what: bit 0 gauge force, bit 1 fermion force.  out = F (kick == 0, out = F)
-// or P -= kick * F (mom != nullptr).
-__global__ void __launch_bounds__(kThreads) force_kernel(Geom g, const void* U, const void* X, const void* Y,
-                                                         double beta, double c11, double c12, int what,
-                                                         void* out, void* mom, double kick)
+// F, to out or onto the momenta (P -= kick F)
+__device__ __forceinline__ void force_out(const Geom& g, int p, int mu, int i, const M3& F, void* out, void* mom,
+                                          double kick)
 {
-    int i = blockIdx.x * blockDim.x + threadIdx.x;
-    int p = blockIdx.y >> 2, mu = blockIdx.y & 3;
-    if (i >= g.Vh) return;
-    Walker x = link_coords(g, p, i);
-    M3 F = m3_zero();
-    if (what & 1) F = gauge_force_link(U, g, x, mu, beta, c11, c12);
-    if (what & 2) m3_acc(F, fermion_force_link(U, X, Y, g, x, mu));
     if (mom) {
         M3 P = ld_link(mom, p, mu, i, g.Vh);
         m3_axpy(P, -kick, F);
@@ -175,16 +315,46 @@ __global__ void __launch_bounds__(kThreads) force_kernel(Geom g, const void* U, 
     }
 }
 
-__global__ void __launch_bounds__(kThreads) staple_kernel(Geom g, const void* U, void* A1out, void* A2out)
+// the fermion force, one thread per link (add: onto the force in out)
+__global__ void __launch_bounds__(kThreads) fermion_force_kernel(Geom g, const void* U, const void* X, const void* Y,
+                                                                 int add, void* out, void* mom, double kick)
 {
     int i = blockIdx.x * blockDim.x + threadIdx.x;
     int p = blockIdx.y >> 2, mu = blockIdx.y & 3;
     if (i >= g.Vh) return;
-    Walker x = link_coords(g, p, i);
-    M3 A1, A2;
-    staples(U, g, x, mu, A1, A2);
-    st_link(A1out, p, mu, i, g.Vh, A1);
-    st_link(A2out, p, mu, i, g.Vh, A2);
+    M3 F = fermion_force_link(U, X, Y, g, eo_coords(g, p, i), p, mu);
+    if (add) m3_acc(F, ld_link(out, p, mu, i, g.Vh));
+    force_out(g, p, mu, i, F, out, mom, kick);
+}
+
+// The gauge force F_g = -i (beta/12) (U V - (U V)^dag), V = c11 A1 + c12 A2
+// (Fermions.cpp:372-384).
+__global__ void __launch_bounds__(kSideThreads, 2) gauge_force_kernel(Geom g, const void* U, double beta, double c11,
+                                                                      double c12, void* out, void* mom, double kick)
+{
+    __shared__ SideSum sum;
+    const int i = blockIdx.x * 32 + (threadIdx.x & 31), p = blockIdx.y >> 2, mu = blockIdx.y & 3;
+    M3 S;
+    side_staples(U, g, eo_coords(g, p, min(i, g.Vh - 1)), p, mu, c11, c12, S, S);
+    sum_sides(sum, S);
+    if (threadIdx.x >= 32 || i >= g.Vh) return;
+    const M3 F = antiherm_force(m3_mul_adj(ld_link(U, p, mu, i, g.Vh), side_sum(sum)), beta / 12.0);
+    force_out(g, p, mu, i, F, out, mom, kick);
+}
+
+// A1 (plaquette staples) and A2 (rectangle staples), walked from x + mu back to x
+__global__ void __launch_bounds__(kSideThreads, 2) staple_kernel(Geom g, const void* U, void* A1out, void* A2out)
+{
+    __shared__ SideSum sum;
+    const int i = blockIdx.x * 32 + (threadIdx.x & 31), p = blockIdx.y >> 2, mu = blockIdx.y & 3;
+    M3 S[2];
+    side_staples<true>(U, g, eo_coords(g, p, min(i, g.Vh - 1)), p, mu, 1.0, 1.0, S[0], S[1]);
+#pragma unroll
+    for (int k = 0; k < 2; ++k) {
+        sum_sides(sum, S[k]);
+        if (threadIdx.x < 32 && i < g.Vh) st_link(k == 0 ? A1out : A2out, p, mu, i, g.Vh, m3_adj(side_sum(sum)));
+        __syncthreads();
+    }
 }
 
 // Fermions.cpp:699-723, 984-994: U <- exp(i eps P) U.  check: the production
@@ -225,8 +395,8 @@ __global__ void link_update_kernel(Geom g, void* U, const void* P, double eps, i
 // deterministic FP64 reductions: fixed grid, per-block partials, one final
 // block summing the partials in order
 // ---------------------------------------------------------------------------
-constexpr int kRedBlocks = 1024;
-constexpr int kRedThreads = 256;
+constexpr int kRedBlocks = 1184;  // eight per SM; launch_reduce's partial array holds 2048
+constexpr int kRedThreads = 128;
 
 __device__ __forceinline__ double block_reduce(double v, double* sm)
 {
@@ -242,45 +412,62 @@ __device__ __forceinline__ double block_reduce(double v, double* sm)
     return r;
 }
 
-// per link: Re Tr P^2 (Fermions.cpp:662-678); gauge action density
-// -(beta/3)(c11 ReTr(U A1)/4 + c12 ReTr(U A2)/6) (Lattice.cpp:759-781);
-// ReTr(U A1)/3 (Lattice.cpp:784-804).  RED_DOT: Re<a, b> over spinors.
-__global__ void __launch_bounds__(kRedThreads) reduce_kernel(Geom g, int kind, const void* A, const void* B,
-                                                             double beta, double c11, double c12, double* partial)
+// The plane loops of site x, directions mu < nu: Re Tr of the plaquette and
+// (RECT) of the two rectangles that start there, each loop of the lattice
+// once.  The staple sums of the reference count a plaquette at each of its
+// four links and a rectangle at each of its six, so that
+// sum_links Re Tr(U A1) = 4 sum P and sum_links Re Tr(U A2) = 6 sum R; counting
+// loops takes 8 products per site and plane instead of 37 per link and plane.
+template <bool RECT>
+__device__ __forceinline__ void plane_loops(const PlaneSite& s, int mu, int nu, double& plaq, double& rect)
+{
+    const M3 Un = plane_link(s, nu, 0, 0), Um = plane_link(s, mu, 0, 0);
+    const M3 mn = m3_mul(Um, plane_link(s, nu, 1, 0));   // x -> x + mu -> x + mu + nu
+    const M3 nm = m3_mul(Un, plane_link(s, mu, 0, 1));   // x -> x + nu -> x + mu + nu
+    plaq = m3_retr_adj(mn, nm);
+    rect = 0.0;
+    if constexpr (RECT) {
+        // 2 x 1: U_mu(x) U_mu(x + mu) U_nu(x + 2 mu) against nm U_mu(x + mu + nu)
+        M3 a = m3_mul(Um, m3_mul(plane_link(s, mu, 1, 0), plane_link(s, nu, 2, 0)));
+        rect = m3_retr_adj(a, m3_mul(nm, plane_link(s, mu, 1, 1)));
+        // 1 x 2: mn U_nu(x + mu + nu) against U_nu(x) U_nu(x + nu) U_mu(x + 2 nu)
+        a = m3_mul(Un, m3_mul(plane_link(s, nu, 0, 1), plane_link(s, mu, 0, 2)));
+        rect += m3_retr_adj(m3_mul(mn, plane_link(s, nu, 1, 1)), a);
+    }
+}
+
+// RED_TRP2: Re Tr P^2 of every link (Fermions.cpp:662-678); RED_ACTION:
+// -(beta/3) (c11 P + c12 R) (Lattice.cpp:759-781) and RED_PLAQ: 4 P / 3
+// (Lattice.cpp:784-804) of every site and plane; RED_DOT: Re<a, b> over spinors.
+template <int KIND>
+__global__ void __launch_bounds__(kRedThreads) reduce_kernel(Geom g, const void* A, const void* B, double beta,
+                                                             double c11, double c12, double* partial)
 {
     __shared__ double sm[32];
     double acc = 0.0;
-    const long nlinks = 4L * g.V;
-    if (kind == RED_DOT) {
+    const long first = blockIdx.x * (long)blockDim.x + threadIdx.x, step = (long)gridDim.x * blockDim.x;
+    if constexpr (KIND == RED_DOT) {
         const double* a = (const double*)A;
         const double* b = (const double*)B;
         const long n = 6L * g.V;
-        for (long k = blockIdx.x * (long)blockDim.x + threadIdx.x; k < n; k += (long)gridDim.x * blockDim.x)
-            acc += a[k] * b[k];
+        for (long k = first; k < n; k += step) acc += a[k] * b[k];
+    } else if constexpr (KIND == RED_TRP2) {
+        const long nlinks = 4L * g.V;
+        for (long l = first; l < nlinks; l += step) {
+            const int pm = (int)(l / g.Vh), i = (int)(l - (long)pm * g.Vh);
+            const M3 P = ld_link(A, pm >> 2, pm & 3, i, g.Vh);
+            acc += m3_retr(P, P);
+        }
     } else {
-        for (long l = blockIdx.x * (long)blockDim.x + threadIdx.x; l < nlinks; l += (long)gridDim.x * blockDim.x) {
-            int pm = (int)(l / g.Vh);
-            int i = (int)(l - (long)pm * g.Vh);
-            int p = pm >> 2, mu = pm & 3;
-            if (kind == RED_TRP2) {
-                M3 P = ld_link(A, p, mu, i, g.Vh);
-                acc += m3_tr(m3_mul(P, P)).re;
-            } else {
-                Walker x = link_coords(g, p, i);
-                M3 A1, A2;
-                if (kind == RED_PLAQ)
-                    staples<false>(A, g, x, mu, A1, A2);  // the plaquette staples only
-                else
-                    staples(A, g, x, mu, A1, A2);
-                M3 Ux = link_at(A, g, x, mu);
-                double plaq = m3_tr(m3_mul(Ux, A1)).re;
-                if (kind == RED_PLAQ) {
-                    acc += plaq / 3.0;
-                } else {
-                    double rect = m3_tr(m3_mul(Ux, A2)).re;
-                    acc += -(beta / 3.0) * (c11 * plaq / 4.0 + c12 * rect / 6.0);
-                }
-            }
+        const long n = 12L * g.Vh;  // (parity, plane, site)
+        for (long l = first; l < n; l += step) {
+            const int pp = (int)(l / g.Vh), i = (int)(l - (long)pp * g.Vh);
+            const int p = pp >= 6 ? 1 : 0, plane = pp - 6 * p;  // (0,1) (0,2) (0,3) (1,2) (1,3) (2,3)
+            const int mu = plane < 3 ? 0 : (plane < 5 ? 1 : 2), nu = plane < 3 ? plane + 1 : (plane < 5 ? plane - 1 : 3);
+            const PlaneSite s = plane_site(A, g, eo_coords(g, p, i), p, mu, nu);
+            double P, R;
+            plane_loops<KIND == RED_ACTION>(s, mu, nu, P, R);
+            acc += KIND == RED_PLAQ ? (4.0 / 3.0) * P : -(beta / 3.0) * (c11 * P + c12 * R);
         }
     }
     double r = block_reduce(acc, sm);
@@ -298,11 +485,15 @@ __global__ void reduce_final(const double* partial, int n, double* out)
 
 }  // namespace
 
+// what: bit 0 gauge force, bit 1 fermion force; out = F, or P -= kick F (mom)
 cudaError_t launch_force(const Geom& g, const void* U, const void* X, const void* Y, double beta, double c11,
                          double c12, int what, void* out, void* mom, double kick, cudaStream_t s)
 {
-    force_kernel<<<dim3((g.Vh + kThreads - 1) / kThreads, 8), kThreads, 0, s>>>(g, U, X, Y, beta, c11, c12, what,
-                                                                                 out, mom, kick);
+    if (what & 1)
+        gauge_force_kernel<<<dim3((g.Vh + 31) / 32, 8), kSideThreads, 0, s>>>(g, U, beta, c11, c12, out, mom, kick);
+    if (what & 2)
+        fermion_force_kernel<<<dim3((g.Vh + kThreads - 1) / kThreads, 8), kThreads, 0, s>>>(
+            g, U, X, Y, (what & 1) && !mom, out, mom, kick);
     return cudaGetLastError();
 }
 
@@ -376,10 +567,22 @@ __device__ __forceinline__ void quat_su2(const double (&q)[4], Cx<double> (&m)[4
     m[3] = {q[0], -q[3]};
 }
 
-__device__ void hb_subgroup(HbRng& r, M3& U, const M3& A, int i, int j, double beta)
+// element (a, b) of U S^dag
+__device__ __forceinline__ Cx<double> hb_block(const M3& U, const M3& S, int a, int b)
 {
-    const M3 UA = m3_mul(U, A);
-    const Cx<double> b0 = UA.e[i * 3 + i], b1 = UA.e[i * 3 + j], b2 = UA.e[j * 3 + i], b3 = UA.e[j * 3 + j];
+    Cx<double> s;
+    cfma_bc<true>(s, U.e[a * 3], S.e[b * 3]);
+    cfma_bc<false>(s, U.e[a * 3 + 1], S.e[b * 3 + 1]);
+    cfma_bc<false>(s, U.e[a * 3 + 2], S.e[b * 3 + 2]);
+    return s;
+}
+
+// one subgroup (rows I, J) of the link U with staple sum A = S^dag
+template <int i, int j>
+__device__ __forceinline__ void hb_subgroup(HbRng& r, M3& U, const M3& S, double beta)
+{
+    const Cx<double> b0 = hb_block(U, S, i, i), b1 = hb_block(U, S, i, j), b2 = hb_block(U, S, j, i),
+                     b3 = hb_block(U, S, j, j);
     const double w0 = 0.5 * (b0.re + b3.re), w1 = 0.5 * (b1.im + b2.im);
     const double w2 = 0.5 * (b1.re - b2.re), w3 = 0.5 * (b0.im - b3.im);
     const double a = sqrt(w0 * w0 + w1 * w1 + w2 * w2 + w3 * w3);
@@ -403,51 +606,75 @@ __device__ void hb_subgroup(HbRng& r, M3& U, const M3& A, int i, int j, double b
         R[2] = cadd(cmul(X[2], Wd[0]), cmul(X[3], Wd[2]));
         R[3] = cadd(cmul(X[2], Wd[1]), cmul(X[3], Wd[3]));
     }
-    M3 E = m3_id();
-    E.e[i * 3 + i] = R[0];
-    E.e[i * 3 + j] = R[1];
-    E.e[j * 3 + i] = R[2];
-    E.e[j * 3 + j] = R[3];
-    U = m3_mul(E, U);
+#pragma unroll
+    for (int k = 0; k < 3; ++k) {  // rows i and j of R U
+        const Cx<double> ui = U.e[i * 3 + k], uj = U.e[j * 3 + k];
+        cfma<true>(U.e[i * 3 + k], R[0], ui);
+        cfma<false>(U.e[i * 3 + k], R[1], uj);
+        cfma<true>(U.e[j * 3 + k], R[2], ui);
+        cfma<false>(U.e[j * 3 + k], R[3], uj);
+    }
 }
 
-__global__ void __launch_bounds__(128) heatbath_kernel(Geom g, void* U, int mu, int colour, double beta, double c11,
-                                                       double c12, unsigned long long seed, int sweep)
+// site k of the V / 8 sites of one colour of direction mu, in an order that
+// keeps t fastest: the colour fixes x_mu mod 2 and one other coordinate (t, or
+// z for mu = t) mod 4 given the rest
+__device__ __forceinline__ Coord hb_site(const Geom& g, int mu, int colour, int k)
 {
-    const int s = blockIdx.x * blockDim.x + threadIdx.x;
-    if (s >= g.V) return;
-    Walker x;
-    int rest = s;
-    x.x[3] = rest % g.L[3];
-    rest /= g.L[3];
-    x.x[2] = rest % g.L[2];
-    rest /= g.L[2];
-    x.x[1] = rest % g.L[1];
-    x.x[0] = rest / g.L[1];
-    int sum = 0;
+    const int d = mu == 3 ? 2 : 3;  // the coordinate that the sum fixes mod 4
+    int x[4], rest = k, sum = 0;
 #pragma unroll
-    for (int nu = 0; nu < 4; ++nu)
-        if (nu != mu) sum += x.x[nu];
-    if ((x.x[mu] & 1) * 4 + (sum & 3) != colour) return;
-    M3 A1, A2;
-    staples(U, g, x, mu, A1, A2);
-    M3 A = m3_zero();
-    m3_axpy(A, c11, A1);
-    m3_axpy(A, c12, A2);
-    const int p = (x.x[0] + x.x[1] + x.x[2] + x.x[3]) & 1, i = s >> 1;
+    for (int nu = 3; nu >= 0; --nu) {
+        const int n = nu == mu ? g.L[nu] / 2 : (nu == d ? g.L[nu] / 4 : g.L[nu]);
+        x[nu] = rest % n;
+        rest /= n;
+        if (nu == mu) x[nu] = 2 * x[nu] + (colour >> 2);
+        else if (nu != d) sum += x[nu];
+    }
+    const int r = ((colour & 3) - sum) & 3;
+    if (mu == 3) x[2] = 4 * x[2] + r;
+    else x[3] = 4 * x[3] + r;
+    Coord c;
+#pragma unroll
+    for (int nu = 0; nu < 4; ++nu) c.x[nu] = x[nu];
+    c.lex = ((x[0] * g.L[1] + x[1]) * g.L[2] + x[2]) * g.L[3] + x[3];
+    return c;
+}
+
+// Only the colour's links have threads (one link in eight of a thread per site
+// left every warp an eighth full): six warps share the staples of 32 of them (a
+// launch at 16^4 has 8192 links, 55 per SM, and their staples are a chain of 66
+// products), then one warp updates them: 112 -> 28 us a launch at 16^4, where
+// the three subgroups' sampling loops in one warp are now most of it.
+__global__ void __launch_bounds__(kSideThreads, 2) heatbath_kernel(Geom g, void* U, int mu, int colour, double beta,
+                                                                   double c11, double c12, unsigned long long seed,
+                                                                   int sweep)
+{
+    __shared__ SideSum sum;
+    const int k = blockIdx.x * 32 + (threadIdx.x & 31), n = g.V / 8;
+    const Coord c = hb_site(g, mu, colour, min(k, n - 1));
+    const int p = (c.x[0] + c.x[1] + c.x[2] + c.x[3]) & 1, i = c.lex >> 1;
+    M3 S;
+    side_staples(U, g, c, p, mu, c11, c12, S, S);
+    sum_sides(sum, S);
+    if (threadIdx.x >= 32 || k >= n) return;
+    S = side_sum(sum);
     M3 u = ld_link(U, p, mu, i, g.Vh);
-    const int sub[3][2] = {{0, 1}, {0, 2}, {1, 2}};
-#pragma unroll 1
-    for (int k = 0; k < 3; ++k) {
-        HbRng r;
-        r.key = make_uint2((unsigned)seed, (unsigned)(seed >> 32));
-        r.link = (unsigned)(s * 4 + mu);
-        r.sweep = (unsigned)sweep;
-        r.tag = 0x48420000u + (unsigned)k;
+    HbRng r;
+    r.key = make_uint2((unsigned)seed, (unsigned)(seed >> 32));
+    r.link = (unsigned)(c.lex * 4 + mu);
+    r.sweep = (unsigned)sweep;
+    auto restart = [&](int sub) {
+        r.tag = 0x48420000u + (unsigned)sub;
         r.draw = 0;
         r.have = 0;
-        hb_subgroup(r, u, A, sub[k][0], sub[k][1], beta);
-    }
+    };
+    restart(0);
+    hb_subgroup<0, 1>(r, u, S, beta);
+    restart(1);
+    hb_subgroup<0, 2>(r, u, S, beta);
+    restart(2);
+    hb_subgroup<1, 2>(r, u, S, beta);
     st_link(U, p, mu, i, g.Vh, u);
 }
 
@@ -457,7 +684,7 @@ cudaError_t launch_heatbath(const Geom& g, void* U, double beta, double c11, dou
     for (int sw = sweep0; sw < sweep0 + nsweeps; ++sw)
         for (int mu = 0; mu < 4; ++mu)
             for (int col = 0; col < 8; ++col)
-                heatbath_kernel<<<(g.V + 127) / 128, 128, 0, s>>>(g, U, mu, col, beta, c11, c12, seed, sw);
+                heatbath_kernel<<<(g.V / 8 + 31) / 32, kSideThreads, 0, s>>>(g, U, mu, col, beta, c11, c12, seed, sw);
     return cudaGetLastError();
 }
 
@@ -479,7 +706,7 @@ cudaError_t launch_link_axpy(const Geom& g, void* Y, double a, const void* X, cu
 
 cudaError_t launch_staples(const Geom& g, const void* U, void* A1, void* A2, cudaStream_t s)
 {
-    staple_kernel<<<dim3((g.Vh + kThreads - 1) / kThreads, 8), kThreads, 0, s>>>(g, U, A1, A2);
+    staple_kernel<<<dim3((g.Vh + 31) / 32, 8), kSideThreads, 0, s>>>(g, U, A1, A2);
     return cudaGetLastError();
 }
 
@@ -494,7 +721,11 @@ cudaError_t launch_link_update(const Geom& g, void* U, const void* P, double eps
 cudaError_t launch_reduce(const Geom& g, int kind, const void* A, const void* B, double beta, double c11,
                           double c12, double* partial, double* out, cudaStream_t s)
 {
-    reduce_kernel<<<kRedBlocks, kRedThreads, 0, s>>>(g, kind, A, B, beta, c11, c12, partial);
+    const auto k = kind == RED_TRP2     ? reduce_kernel<RED_TRP2>
+                   : kind == RED_ACTION ? reduce_kernel<RED_ACTION>
+                   : kind == RED_PLAQ   ? reduce_kernel<RED_PLAQ>
+                                        : reduce_kernel<RED_DOT>;
+    k<<<kRedBlocks, kRedThreads, 0, s>>>(g, A, B, beta, c11, c12, partial);
     reduce_final<<<1, 1024, 0, s>>>(partial, kRedBlocks, out);
     return cudaGetLastError();
 }

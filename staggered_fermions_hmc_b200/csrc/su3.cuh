@@ -28,52 +28,119 @@ __device__ __forceinline__ M3 m3_id()
     return m;
 }
 
-// a b
+// s (+)= a b, a conj(b), conj(a) b as FMA chains (FIRST: s = instead of s +=)
+template <bool FIRST>
+__device__ __forceinline__ void cfma(Cx<double>& s, const Cx<double>& a, const Cx<double>& b)
+{
+    s.re = FIRST ? a.re * b.re : fma(a.re, b.re, s.re);
+    s.im = FIRST ? a.re * b.im : fma(a.re, b.im, s.im);
+    s.re = fma(-a.im, b.im, s.re);
+    s.im = fma(a.im, b.re, s.im);
+}
+template <bool FIRST>
+__device__ __forceinline__ void cfma_bc(Cx<double>& s, const Cx<double>& a, const Cx<double>& b)
+{
+    s.re = FIRST ? a.re * b.re : fma(a.re, b.re, s.re);
+    s.im = FIRST ? a.im * b.re : fma(a.im, b.re, s.im);
+    s.re = fma(a.im, b.im, s.re);
+    s.im = fma(-a.re, b.im, s.im);
+}
+template <bool FIRST>
+__device__ __forceinline__ void cfma_ac(Cx<double>& s, const Cx<double>& a, const Cx<double>& b)
+{
+    s.re = FIRST ? a.re * b.re : fma(a.re, b.re, s.re);
+    s.im = FIRST ? a.re * b.im : fma(a.re, b.im, s.im);
+    s.re = fma(a.im, b.im, s.re);
+    s.im = fma(-a.im, b.re, s.im);
+}
+
+// The products as 108 FMAs: a complex multiply followed by an add costs a
+// third more instructions.
+// o = a b (ACC: o += a b)
+template <bool ACC>
+__device__ __forceinline__ void m3_mul_to(M3& o, const M3& a, const M3& b)
+{
+#pragma unroll
+    for (int i = 0; i < 3; ++i)
+#pragma unroll
+        for (int j = 0; j < 3; ++j) {
+            Cx<double>& s = o.e[i * 3 + j];
+            cfma<!ACC>(s, a.e[i * 3], b.e[j]);
+            cfma<false>(s, a.e[i * 3 + 1], b.e[3 + j]);
+            cfma<false>(s, a.e[i * 3 + 2], b.e[6 + j]);
+        }
+}
+
+// o = a b^dag (ACC: o += a b^dag)
+template <bool ACC>
+__device__ __forceinline__ void m3_mul_adj_to(M3& o, const M3& a, const M3& b)
+{
+#pragma unroll
+    for (int i = 0; i < 3; ++i)
+#pragma unroll
+        for (int j = 0; j < 3; ++j) {
+            Cx<double>& s = o.e[i * 3 + j];
+            cfma_bc<!ACC>(s, a.e[i * 3], b.e[j * 3]);
+            cfma_bc<false>(s, a.e[i * 3 + 1], b.e[j * 3 + 1]);
+            cfma_bc<false>(s, a.e[i * 3 + 2], b.e[j * 3 + 2]);
+        }
+}
+
+// o = a^dag b (ACC: o += a^dag b)
+template <bool ACC>
+__device__ __forceinline__ void m3_adj_mul_to(M3& o, const M3& a, const M3& b)
+{
+#pragma unroll
+    for (int i = 0; i < 3; ++i)
+#pragma unroll
+        for (int j = 0; j < 3; ++j) {
+            Cx<double>& s = o.e[i * 3 + j];
+            cfma_ac<!ACC>(s, a.e[i], b.e[j]);
+            cfma_ac<false>(s, a.e[3 + i], b.e[3 + j]);
+            cfma_ac<false>(s, a.e[6 + i], b.e[6 + j]);
+        }
+}
+
 __device__ __forceinline__ M3 m3_mul(const M3& a, const M3& b)
 {
     M3 o;
-#pragma unroll
-    for (int i = 0; i < 3; ++i)
-#pragma unroll
-        for (int j = 0; j < 3; ++j) {
-            Cx<double> s = cmul(a.e[i * 3], b.e[j]);
-            s = cadd(s, cmul(a.e[i * 3 + 1], b.e[3 + j]));
-            s = cadd(s, cmul(a.e[i * 3 + 2], b.e[6 + j]));
-            o.e[i * 3 + j] = s;
-        }
+    m3_mul_to<false>(o, a, b);
     return o;
 }
 
-// a b^dag
 __device__ __forceinline__ M3 m3_mul_adj(const M3& a, const M3& b)
 {
     M3 o;
-#pragma unroll
-    for (int i = 0; i < 3; ++i)
-#pragma unroll
-        for (int j = 0; j < 3; ++j) {
-            Cx<double> s = cmul(a.e[i * 3], cconj(b.e[j * 3]));
-            s = cadd(s, cmul(a.e[i * 3 + 1], cconj(b.e[j * 3 + 1])));
-            s = cadd(s, cmul(a.e[i * 3 + 2], cconj(b.e[j * 3 + 2])));
-            o.e[i * 3 + j] = s;
-        }
+    m3_mul_adj_to<false>(o, a, b);
     return o;
 }
 
-// a^dag b
 __device__ __forceinline__ M3 m3_adj_mul(const M3& a, const M3& b)
 {
     M3 o;
+    m3_adj_mul_to<false>(o, a, b);
+    return o;
+}
+
+// Re tr(a b), Re tr(a b^dag)
+__device__ __forceinline__ double m3_retr(const M3& a, const M3& b)
+{
+    double s = 0.0;
 #pragma unroll
     for (int i = 0; i < 3; ++i)
 #pragma unroll
-        for (int j = 0; j < 3; ++j) {
-            Cx<double> s = cmul(cconj(a.e[i]), b.e[j]);
-            s = cadd(s, cmul(cconj(a.e[3 + i]), b.e[3 + j]));
-            s = cadd(s, cmul(cconj(a.e[6 + i]), b.e[6 + j]));
-            o.e[i * 3 + j] = s;
+        for (int k = 0; k < 3; ++k) {
+            s = fma(a.e[i * 3 + k].re, b.e[k * 3 + i].re, s);
+            s = fma(-a.e[i * 3 + k].im, b.e[k * 3 + i].im, s);
         }
-    return o;
+    return s;
+}
+__device__ __forceinline__ double m3_retr_adj(const M3& a, const M3& b)
+{
+    double s = 0.0;
+#pragma unroll
+    for (int k = 0; k < 9; ++k) s = fma(a.e[k].im, b.e[k].im, fma(a.e[k].re, b.e[k].re, s));
+    return s;
 }
 
 __device__ __forceinline__ M3 m3_adj(const M3& a)

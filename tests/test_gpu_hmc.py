@@ -499,3 +499,41 @@ def test_kernel_timing_leaves_fields_unchanged(sfh, orc):
         assert np.array_equal(lat.download_momenta(), P)
     finally:
         lat.close()
+
+
+@pytest.mark.parametrize("dims", [(2, 2, 2, 2), (2, 6, 4, 2), (6, 2, 2, 10), (4, 6, 10, 6)])
+@pytest.mark.parametrize("unitary", [True, False])
+def test_staple_kernels_at_odd_sizes(sfh, orc, dims, unitary):
+    """The six-sided staple kernels where a block's 32 links are not full and a
+    step of two sites wraps onto itself (extent 2), on SU(3) links and on
+    general matrices (no row is taken for granted): staples, forces, action and
+    plaquette against the oracle's walks.  FP64 sums of products of up to six
+    matrices: 1e-12 relative, the operators' tolerance."""
+    U = orc.random_gauge(dims, 0.6, 71)
+    if not unitary:
+        U = U + 0.1 * np.random.default_rng(72).standard_normal(U.size)
+    X, Y = orc.random_spinor(dims, 73), orc.random_spinor(dims, 74)
+    lat = sfh.Lattice(dims, 0.2, 4.2)
+    lat.upload_gauge(U)
+    A1, A2 = lat.staples()
+    R1, R2 = orc.staples(dims, U)
+    assert rel(A1, R1) < 1e-12 and rel(A2, R2) < 1e-12
+    Fg, Ff = orc.gauge_force(dims, 4.2, U), orc.fermion_force(dims, U, X, Y)
+    assert rel(lat.compute_gauge_only_force_field(), Fg) < 1e-12
+    assert rel(lat.compute_full_force_field(X, Y), Fg + Ff) < 1e-12
+    assert abs(lat.compute_action() - orc.action(dims, 4.2, U)) < 1e-12 * abs(orc.action(dims, 4.2, U))
+    assert abs(lat.compute_avg_plaq() - orc.avg_plaq(dims, U)) < 1e-12 * abs(orc.avg_plaq(dims, U))
+    lat.close()
+
+
+@pytest.mark.parametrize("dims", [(8, 4, 4, 12), (4, 12, 8, 4), (4, 8, 4, 8)])
+def test_heatbath_at_unequal_extents(sfh, orc, dims):
+    """The heatbath's threads enumerate the links of one colour only: every
+    link of every direction is updated once per sweep, with its own uniforms,
+    whatever extents the colours run over (as test_heatbath_vs_oracle)."""
+    U = orc.random_gauge(dims, 0.6, 193)
+    lat = sfh.Lattice(dims, 0.1, 4.2)
+    lat.upload_gauge(U)
+    lat.heatbath_update(n_sweeps=2, seed=29, sweep0=1)
+    assert rel(lat.download_gauge(), orc.heatbath(dims, 4.2, U, seed=29, nsweeps=2, sweep0=1)) < 1e-12
+    lat.close()
