@@ -347,7 +347,7 @@ int sfh_batch_autotune(sfh_batch* batch, int probe_iters, int* best_width);
  * (width, tiles and staging all 0, the default: small batches, at most 8 RHS
  * per system and 1024 site-lanes per SM and parity, fewer for the wider
  * precisions, run the whole solve in one dataflow launch, whose sums are added
- * in another order; the rest staging 0):
+ * in another order; the rest take a schedule by their size):
  * 0 links read directly per RHS group; 1 staged in shared memory per work
  * item with asynchronous copies; 2 system-blocked: one block per tile serves
  * every RHS of its system in groups of the RHS-block width, the tile's links

@@ -2059,10 +2059,75 @@ static cudaError_t flow_solve(CgWorkspace& w, const CgArgs& a, cudaStream_t stre
     return cudaSuccess;
 }
 
+// The per-phase kernels' schedule when the caller leaves all of it open
+// (widths, tiles per work item, staging; 0: as below).  It never changes the
+// mixed precisions' results.
+//
+// Several RHS or systems: groups of two, in FP16 of four in the first hop; from
+// 400000 sites x RHS on the reliable updates in the lane-list kernels (two more
+// launches; FP16 and FP32-12: the BF16 hop gains less from their registers, the
+// FP32 18-real one is a third slower without them inline).  Against groups of
+// eight and four with inline updates, ms: 20 uneven systems, 94 RHS, FP16 225 ->
+// 192, FP32 277 -> 230, BF16 262 -> 232; 16^4 with 8 RHS FP16 28.6 -> 23.6; below
+// the line, 20^4 with 2 RHS, the lane lists would take 21.3 for 20.2.
+//
+// One RHS: the tiles per item and the staging of least cost, counted in tile
+// times of an SM: B = ceil(items / SMs) blocks of `tiles` tiles each, four for
+// every wave of resident blocks (launch, descriptors, partial last wave) and
+// three for the two more kernels of the lane lists.  Against two tiles and
+// inline updates, m 0.2, ms: FP32 24^3 32 17.3 -> 14.4, 24^4 13.3 -> 12.4 and
+// 32^3 64 77.9 -> 71.6; FP16 28^4 20.4 -> 19.3, 32^4 (m 0.1) 61.0 -> 51.1; BF16
+// 32^3 64 76.4 -> 65.5.  On smaller lattices the 16-bit storages gained nothing
+// (18 22 26 30: FP16 10.9 against 11.3), nor did FP64 and FP32 18-real anywhere.
+struct AutoSchedule {
+    int nb1 = 0, nb2 = 0, tpi = 0, stage = 0;
+};
+
+static AutoSchedule auto_schedule(const CgWorkspace& w)
+{
+    AutoSchedule s;
+    if (w.prec == SFH_PREC_F64) return s;
+    const bool f16 = w.prec == SFH_PREC_F16, f32 = w.prec == SFH_PREC_F32;
+    if (w.nlanes > 2) {
+        if (w.auto_nb > 0) return s;  // a pair of masses keeps its own widths
+        long work = 0;
+        int most = 1;
+        for (const CgSys& S : w.sys) {
+            work += (long)S.g.V * S.nrhs;
+            most = std::max(most, S.nrhs);
+        }
+        s.nb1 = default_nb(most, f16 ? 4 : 2);
+        s.nb2 = default_nb(most, 2);
+        s.stage = (f16 || f32) && work >= 400000 ? 4 : 0;
+        return s;
+    }
+    if (w.prec == SFH_PREC_F32_18) return s;
+    const int sms = std::max(1, w.num_sms), tiles = 2 * w.sys[0].ntq;
+    if (!f32 && tiles < (f16 ? 2000 : 4000)) return s;
+    int best = 1 << 30;
+    for (int stage : {0, 4})
+        for (int tpi : {1, 2, 4, 8, 16}) {
+            const int occ = stage == 0 ? (f16 ? HopOcc<GP_F16_12, SP_F16, 1, true, true>::v
+                                              : HopOcc<GP_F32_12, SP_F32, 1, true, true>::v)
+                                       : (f16 ? HopOcc<GP_F16_12, SP_F16, 1, true, false>::v
+                                              : HopOcc<GP_F32_12, SP_F32, 1, true, false>::v);
+            const int items = 2 * ((tiles / 2 + tpi - 1) / tpi), B = (items + sms - 1) / sms;
+            // a block alone on its SM does not keep it busy
+            const int cost = std::max(B, 2) * tpi + 4 * ((B + occ - 1) / occ) + (stage ? 3 : 0);
+            if (cost < best || (cost == best && stage == s.stage)) {
+                best = cost;
+                s.tpi = tpi;
+                s.stage = stage;
+            }
+        }
+    return s;
+}
+
 // Solve every lane of a built workspace.  nb1 / nb2: RHS-block widths of the
 // two hop kernels (0 = from the largest RHS count); tpi: tiles per block of
 // the iteration kernels (0 = default_tpi); stage: hop kernels stage their
-// links in shared memory (reduced precisions only); prefer_flow: the dataflow
+// links in shared memory (reduced precisions only); all of them 0:
+// auto_schedule; prefer_flow: the dataflow
 // kernel where the systems suit it, whatever the schedule.  Returns a cudaError.
 static cudaError_t workspace_solve(CgWorkspace& w, double tol, int maxit, double delta, int nb1, int nb2,
                                    int tpi, int stage, cudaStream_t stream, PhaseTimes* timing = nullptr,
@@ -2074,12 +2139,20 @@ static cudaError_t workspace_solve(CgWorkspace& w, double tol, int maxit, double
     // without an explicit schedule, systems that fit the SMs' shared memory
     // take the dataflow kernel (flow_plan says where the line lies)
     bool flow = false;
-    if (!timing && (prefer_flow || (nb1 <= 0 && nb2 <= 0 && tpi <= 0 && stage == 0))) {
+    const bool open = nb1 <= 0 && nb2 <= 0 && tpi <= 0 && stage == 0;
+    if (!timing && (prefer_flow || open)) {
         if (w.flow.state == 0) {
             const cudaError_t fe = flow_prepare(w);
             if (fe != cudaSuccess) return fe;
         }
         flow = w.flow.state > 0;
+    }
+    if (open && !prefer_flow) {
+        const AutoSchedule s = auto_schedule(w);
+        nb1 = s.nb1;
+        nb2 = s.nb2;
+        tpi = s.tpi;
+        stage = s.stage;
     }
     if (nb1 <= 0) nb1 = w.auto_nb > 0 ? w.auto_nb : default_nb(max_nrhs, f64 ? 2 : 8);
     if (nb2 <= 0) nb2 = w.auto_nb > 0 ? w.auto_nb : default_nb(max_nrhs, f64 ? 2 : 4);
