@@ -16,40 +16,21 @@
 // four matrices instead of six, and the sides' links meet in the L1), and adds
 // the sides through shared memory.  The products are FMA chains (su3.cuh).
 // Measured on the B200, one thread and whole walks per link -> this: gauge
-// force 363 -> 250 us at 16^4, 2196 -> 1399 us at 24^4; staples 2470 -> 1415 us;
+// force 363 -> 247 us at 16^4, 2196 -> 1242 us at 24^4 (1399 with the directions
+// of a site far apart in the grid); staples 2470 -> 1417 us;
 // a heatbath sweep 3.57 -> 0.91 ms at 16^4, 18.1 -> 4.1 ms at 24^4.  It runs at
-// 14 TFLOP/s, 0.4 of the FP64 pipe, latency bound on 12 warps per SM (168
+// 16 TFLOP/s, 0.45 of the FP64 pipe, latency bound on 12 warps per SM (168
 // registers): a third of the stalls are link loads, a fifth each FMA latency
 // and instruction fetch.  A row of the staples per thread (80 registers, 24
 // warps, every link read by three threads) was bound by the L1: 2696 us.
 #include "sfh_internal.h"
-#include "su3.cuh"
+#include "walk.cuh"
 
 namespace sfh {
 
 namespace {
 
 constexpr int kThreads = 128;
-
-__device__ __forceinline__ int coord_of(const Coord& c, int mu)
-{
-    return mu == 0 ? c.x[0] : (mu == 1 ? c.x[1] : (mu == 2 ? c.x[2] : c.x[3]));
-}
-
-__device__ __forceinline__ int extent_of(const Geom& g, int mu)
-{
-    return mu == 0 ? g.L[0] : (mu == 1 ? g.L[1] : (mu == 2 ? g.L[2] : g.L[3]));
-}
-
-// offset of x + k mu, |k| <= 2 <= L
-__device__ __forceinline__ int step_offset(const Geom& g, const Coord& c, int mu, int k)
-{
-    const int L = extent_of(g, mu), x = coord_of(c, mu);
-    int y = x + k;
-    if (y < 0) y += L;
-    if (y >= L) y -= L;
-    return (y - x) * lex_stride(g, mu);
-}
 
 // The links around a site x on one side, +nu or -nu, of direction mu:
 // M(m, k) = U_mu(x + m mu + k side) and D(m, k), the step from x + m mu +
@@ -194,7 +175,9 @@ __device__ __forceinline__ M3 plane_link(const PlaneSite& s, int a, int dm, int 
     return m;
 }
 
-// Blocks of the staple kernels: six warps, one side of 32 links each.
+// Blocks of the staple kernels: six warps, one side of 32 links each.  The
+// parities and directions of a range of sites are adjacent in the grid, so that
+// their links meet in the L2 (a field of 24^4 is larger).
 constexpr int kSides = 6, kSideThreads = 32 * kSides;
 
 // the sides' staples of the block's 32 links: 18 doubles each
@@ -319,8 +302,8 @@ __device__ __forceinline__ void force_out(const Geom& g, int p, int mu, int i, c
 __global__ void __launch_bounds__(kThreads) fermion_force_kernel(Geom g, const void* U, const void* X, const void* Y,
                                                                  int add, void* out, void* mom, double kick)
 {
-    int i = blockIdx.x * blockDim.x + threadIdx.x;
-    int p = blockIdx.y >> 2, mu = blockIdx.y & 3;
+    int i = (blockIdx.x >> 3) * blockDim.x + threadIdx.x;
+    int p = (blockIdx.x >> 2) & 1, mu = blockIdx.x & 3;
     if (i >= g.Vh) return;
     M3 F = fermion_force_link(U, X, Y, g, eo_coords(g, p, i), p, mu);
     if (add) m3_acc(F, ld_link(out, p, mu, i, g.Vh));
@@ -333,7 +316,7 @@ __global__ void __launch_bounds__(kSideThreads, 2) gauge_force_kernel(Geom g, co
                                                                       double c12, void* out, void* mom, double kick)
 {
     __shared__ SideSum sum;
-    const int i = blockIdx.x * 32 + (threadIdx.x & 31), p = blockIdx.y >> 2, mu = blockIdx.y & 3;
+    const int i = (blockIdx.x >> 3) * 32 + (threadIdx.x & 31), p = (blockIdx.x >> 2) & 1, mu = blockIdx.x & 3;
     M3 S;
     side_staples(U, g, eo_coords(g, p, min(i, g.Vh - 1)), p, mu, c11, c12, S, S);
     sum_sides(sum, S);
@@ -346,7 +329,7 @@ __global__ void __launch_bounds__(kSideThreads, 2) gauge_force_kernel(Geom g, co
 __global__ void __launch_bounds__(kSideThreads, 2) staple_kernel(Geom g, const void* U, void* A1out, void* A2out)
 {
     __shared__ SideSum sum;
-    const int i = blockIdx.x * 32 + (threadIdx.x & 31), p = blockIdx.y >> 2, mu = blockIdx.y & 3;
+    const int i = (blockIdx.x >> 3) * 32 + (threadIdx.x & 31), p = (blockIdx.x >> 2) & 1, mu = blockIdx.x & 3;
     M3 S[2];
     side_staples<true>(U, g, eo_coords(g, p, min(i, g.Vh - 1)), p, mu, 1.0, 1.0, S[0], S[1]);
 #pragma unroll
@@ -459,9 +442,12 @@ __global__ void __launch_bounds__(kRedThreads) reduce_kernel(Geom g, const void*
             acc += m3_retr(P, P);
         }
     } else {
-        const long n = 12L * g.Vh;  // (parity, plane, site)
-        for (long l = first; l < n; l += step) {
-            const int pp = (int)(l / g.Vh), i = (int)(l - (long)pp * g.Vh);
+        // block-sized chunks of (parity, plane, site), the parities and planes of
+        // a range of sites in turn, so that they meet in the L2
+        const long chunks = (g.Vh + kRedThreads - 1) / kRedThreads;
+        for (long u = blockIdx.x; u < 12 * chunks; u += gridDim.x) {
+            const int pp = (int)(u % 12), i = (int)(u / 12) * kRedThreads + (int)threadIdx.x;
+            if (i >= g.Vh) continue;
             const int p = pp >= 6 ? 1 : 0, plane = pp - 6 * p;  // (0,1) (0,2) (0,3) (1,2) (1,3) (2,3)
             const int mu = plane < 3 ? 0 : (plane < 5 ? 1 : 2), nu = plane < 3 ? plane + 1 : (plane < 5 ? plane - 1 : 3);
             const PlaneSite s = plane_site(A, g, eo_coords(g, p, i), p, mu, nu);
@@ -490,9 +476,9 @@ cudaError_t launch_force(const Geom& g, const void* U, const void* X, const void
                          double c12, int what, void* out, void* mom, double kick, cudaStream_t s)
 {
     if (what & 1)
-        gauge_force_kernel<<<dim3((g.Vh + 31) / 32, 8), kSideThreads, 0, s>>>(g, U, beta, c11, c12, out, mom, kick);
+        gauge_force_kernel<<<8 * ((g.Vh + 31) / 32), kSideThreads, 0, s>>>(g, U, beta, c11, c12, out, mom, kick);
     if (what & 2)
-        fermion_force_kernel<<<dim3((g.Vh + kThreads - 1) / kThreads, 8), kThreads, 0, s>>>(
+        fermion_force_kernel<<<8 * ((g.Vh + kThreads - 1) / kThreads), kThreads, 0, s>>>(
             g, U, X, Y, (what & 1) && !mom, out, mom, kick);
     return cudaGetLastError();
 }
@@ -706,7 +692,7 @@ cudaError_t launch_link_axpy(const Geom& g, void* Y, double a, const void* X, cu
 
 cudaError_t launch_staples(const Geom& g, const void* U, void* A1, void* A2, cudaStream_t s)
 {
-    staple_kernel<<<dim3((g.Vh + 31) / 32, 8), kSideThreads, 0, s>>>(g, U, A1, A2);
+    staple_kernel<<<8 * ((g.Vh + 31) / 32), kSideThreads, 0, s>>>(g, U, A1, A2);
     return cudaGetLastError();
 }
 

@@ -26,6 +26,8 @@ namespace sfh {
 namespace {
 
 constexpr int kThreads = 128;
+constexpr int kSmearOcc = 3;  // blocks per SM of the smearing kernels
+constexpr int kForceOcc = 2;  // and of the force's
 
 // exp(c proj(G U^dag)) U
 __device__ __forceinline__ bool smear_link(const M3& G, const M3& U, double coef, M3& out)
@@ -55,40 +57,66 @@ __device__ __forceinline__ bool smear_link(const M3& G, const M3& U, double coef
 
 __device__ __forceinline__ int slot_of(int dir, int other) { return other - (other > dir ? 1 : 0); }
 
-__device__ __forceinline__ const void* field(const void* base, int k, const Geom& g)
+__device__ __forceinline__ const double2* field(const void* base, int k, const Geom& g)
 {
-    return (const char*)base + (size_t)k * g.V * 4 * 9 * 16;
+    return (const double2*)base + (size_t)k * g.V * 4 * 9;
 }
 
-// staple from x to x+mu through direction nu with side links from S and the
-// middle link from M: S_nu(x) M_mu(x+nu) S_nu(x+mu)^dag + S_nu(x-nu)^dag M_mu(x-nu) S_nu(x-nu+mu)
-__device__ __forceinline__ M3 staple(const void* Sf, int s_slot, const void* Mf, int m_slot, const Geom& g,
-                                     const Walker& x, int mu, int nu)
+__device__ __forceinline__ M3 ld_at(const double2* f, int Vh, int p, int dir, int lex)
 {
-    Walker xn = x, xm = x, xd = x;
-    walk(g, xn, nu, +1);
-    walk(g, xm, mu, +1);
-    walk(g, xd, nu, -1);
-    Walker xdm = xd;
-    walk(g, xdm, mu, +1);
-    M3 up = m3_mul_adj(m3_mul(link_at(field(Sf, s_slot, g), g, x, nu), link_at(field(Mf, m_slot, g), g, xn, mu)),
-                       link_at(field(Sf, s_slot, g), g, xm, nu));
-    M3 dn = m3_mul(m3_adj_mul(link_at(field(Sf, s_slot, g), g, xd, nu), link_at(field(Mf, m_slot, g), g, xd, mu)),
-                   link_at(field(Sf, s_slot, g), g, xdm, nu));
-    m3_acc(up, dn);
-    return up;
+    const double2* b = f + ((size_t)(p * 4 + dir) * 9) * Vh + (lex >> 1);
+    M3 m;
+#pragma unroll
+    for (int k = 0; k < 9; ++k) {
+        const double2 v = __ldg(b + (size_t)k * Vh);
+        m.e[k] = {v.x, v.y};
+    }
+    return m;
 }
 
-__global__ void __launch_bounds__(kThreads) stout_kernel(Geom g, const void* Uin, void* Uout, double rho, int* err)
+// the same address, which the compiler then does not know for one that it has
+// loaded from: a matrix is read again where it is used again (from the L1)
+// instead of being held in 36 registers
+template <typename T>
+__device__ __forceinline__ const T* again(const T* p)
 {
-    int i = blockIdx.x * blockDim.x + threadIdx.x;
-    int p = blockIdx.y >> 2, mu = blockIdx.y & 3;
+    asm volatile("" : "+l"(p));
+    return p;
+}
+
+// G += the staple from x to x+mu through direction nu with side links from S
+// and the middle link from M: S_nu(x) M_mu(x+nu) S_nu(x+mu)^dag +
+// S_nu(x-nu)^dag M_mu(x-nu) S_nu(x-nu+mu)
+__device__ __forceinline__ void staple_acc(M3& G, const double2* S, const double2* M, const Geom& g, const Coord& c,
+                                           int p, int mu, int nu)
+{
+    const int Vh = g.Vh, x = c.lex, m = step_offset(g, c, mu, 1), u = step_offset(g, c, nu, 1),
+              d = step_offset(g, c, nu, -1);
+    M3 t = m3_mul(ld_at(S, Vh, p, nu, x), ld_at(M, Vh, 1 - p, mu, x + u));
+    m3_mul_adj_to<true>(G, t, ld_at(S, Vh, 1 - p, nu, x + m));
+    t = m3_adj_mul(ld_at(S, Vh, 1 - p, nu, x + d), ld_at(M, Vh, 1 - p, mu, x + d));
+    m3_mul_to<true>(G, t, ld_at(S, Vh, p, nu, x + d + m));
+}
+
+// The smearing kernels: one thread per link (and, in HEX levels 1 and 2, per
+// decorated direction, which keeps one staple sum in flight per thread instead
+// of three).  Chains of dependent FP64 operations bound them, so the warps in
+// flight count: 168 registers (three blocks per SM) with the offsets of a step
+// computed from the coordinates, where runtime-indexed coordinates in local
+// memory took 246 to 255 registers (a fourth block would spill 80 to 190 bytes).
+// With the grid order of link_grid, before -> after: a stout level 84 -> 62 us
+// at 16^4 and 512 -> 288 us at 24^4, a HEX pass 532 -> 340 and 2830 -> 1639 us.
+__global__ void __launch_bounds__(kThreads, kSmearOcc) stout_kernel(Geom g, const void* Uin, void* Uout, double rho,
+                                                                    int* err)
+{
+    int i = (blockIdx.x >> 3) * blockDim.x + threadIdx.x;
+    int p = (blockIdx.x >> 2) & 1, mu = blockIdx.x & 3;
     if (i >= g.Vh) return;
-    Walker x = link_coords(g, p, i);
+    const Coord c = eo_coords(g, p, i);
     M3 C = m3_zero();
 #pragma unroll 1
     for (int nu = 0; nu < 4; ++nu)
-        if (nu != mu) m3_acc(C, staple(Uin, 0, Uin, 0, g, x, mu, nu));
+        if (nu != mu) staple_acc(C, (const double2*)Uin, (const double2*)Uin, g, c, p, mu, nu);
     M3 out;
     if (!smear_link(C, ld_link(Uin, p, mu, i, g.Vh), rho, out)) {
         atomicOr(err, DEV_ERR_DOMAIN);
@@ -97,75 +125,84 @@ __global__ void __launch_bounds__(kThreads) stout_kernel(Geom g, const void* Uin
     st_link(Uout, p, mu, i, g.Vh, out);
 }
 
-// V1(a; r) for the three r != a
-__global__ void __launch_bounds__(kThreads) hex1_kernel(Geom g, const void* U, void* V1, double coef, int* err)
+// the link and the decorated direction of a thread of levels 1 and 2
+struct Decorated {
+    int i, p, mu, slot, nu;
+};
+__device__ __forceinline__ Decorated decorated()
 {
-    int i = blockIdx.x * blockDim.x + threadIdx.x;
-    int p = blockIdx.y >> 2, a = blockIdx.y & 3;
-    if (i >= g.Vh) return;
-    Walker x = link_coords(g, p, i);
-    M3 Ua = ld_link(U, p, a, i, g.Vh);
-#pragma unroll 1
-    for (int r = 0; r < 4; ++r) {
-        if (r == a) continue;
-        M3 out;
-        if (!smear_link(staple(U, 0, U, 0, g, x, a, r), Ua, coef, out)) {
-            atomicOr(err, DEV_ERR_DOMAIN);
-            out = Ua;
-        }
-        st_link((char*)V1 + (size_t)slot_of(a, r) * g.V * 4 * 9 * 16, p, a, i, g.Vh, out);
+    Decorated d;
+    const int chunk = blockIdx.x / 24, k = blockIdx.x - 24 * chunk, pm = k / 3;
+    d.i = chunk * blockDim.x + threadIdx.x;
+    d.p = pm >> 2;
+    d.mu = pm & 3;
+    d.slot = k - 3 * pm;
+    d.nu = d.slot + (d.slot >= d.mu ? 1 : 0);
+    return d;
+}
+
+// V1(a; r) for the three r != a
+__global__ void __launch_bounds__(kThreads, kSmearOcc) hex1_kernel(Geom g, const void* U, void* V1, double coef,
+                                                                   int* err)
+{
+    const Decorated d = decorated();
+    if (d.i >= g.Vh) return;
+    M3 G = m3_zero(), out;
+    staple_acc(G, (const double2*)U, (const double2*)U, g, eo_coords(g, d.p, d.i), d.p, d.mu, d.nu);
+    if (!smear_link(G, ld_link(U, d.p, d.mu, d.i, g.Vh), coef, out)) {
+        atomicOr(err, DEV_ERR_DOMAIN);
+        out = ld_link(U, d.p, d.mu, d.i, g.Vh);
     }
+    st_link((char*)V1 + (size_t)d.slot * g.V * 4 * 9 * 16, d.p, d.mu, d.i, g.Vh, out);
 }
 
 // V2(mu; nu) for the three nu != mu
-__global__ void __launch_bounds__(kThreads) hex2_kernel(Geom g, const void* U, const void* V1, void* V2, double coef,
-                                                        int* err)
+__global__ void __launch_bounds__(kThreads, kSmearOcc) hex2_kernel(Geom g, const void* U, const void* V1, void* V2,
+                                                                   double coef, int* err)
 {
-    int i = blockIdx.x * blockDim.x + threadIdx.x;
-    int p = blockIdx.y >> 2, mu = blockIdx.y & 3;
-    if (i >= g.Vh) return;
-    Walker x = link_coords(g, p, i);
-    M3 Umu = ld_link(U, p, mu, i, g.Vh);
+    const Decorated d = decorated();
+    if (d.i >= g.Vh) return;
+    const Coord c = eo_coords(g, d.p, d.i);
+    M3 G = m3_zero(), out;
 #pragma unroll 1
-    for (int nu = 0; nu < 4; ++nu) {
-        if (nu == mu) continue;
-        M3 G = m3_zero();
-        for (int sg = 0; sg < 4; ++sg) {
-            if (sg == mu || sg == nu) continue;
-            const int r = 6 - mu - nu - sg;  // the direction left out of {mu, nu, sigma}
-            // side links V1(sigma; r), middle link V1(mu; r)
-            m3_acc(G, staple(V1, slot_of(sg, r), V1, slot_of(mu, r), g, x, mu, sg));
-        }
-        M3 out;
-        if (!smear_link(G, Umu, coef, out)) {
-            atomicOr(err, DEV_ERR_DOMAIN);
-            out = Umu;
-        }
-        st_link((char*)V2 + (size_t)slot_of(mu, nu) * g.V * 4 * 9 * 16, p, mu, i, g.Vh, out);
+    for (int sg = 0; sg < 4; ++sg) {
+        if (sg == d.mu || sg == d.nu) continue;
+        const int r = 6 - d.mu - d.nu - sg;  // the direction left out of {mu, nu, sigma}
+        // side links V1(sigma; r), middle link V1(mu; r)
+        staple_acc(G, field(V1, slot_of(sg, r), g), field(V1, slot_of(d.mu, r), g), g, c, d.p, d.mu, sg);
     }
+    if (!smear_link(G, ld_link(U, d.p, d.mu, d.i, g.Vh), coef, out)) {
+        atomicOr(err, DEV_ERR_DOMAIN);
+        out = ld_link(U, d.p, d.mu, d.i, g.Vh);
+    }
+    st_link((char*)V2 + (size_t)d.slot * g.V * 4 * 9 * 16, d.p, d.mu, d.i, g.Vh, out);
 }
 
 // U'_mu from the V2 staples (in place: level 3 reads U only at its own link)
-__global__ void __launch_bounds__(kThreads) hex3_kernel(Geom g, void* U, const void* V2, double coef, int* err)
+__global__ void __launch_bounds__(kThreads, kSmearOcc) hex3_kernel(Geom g, void* U, const void* V2, double coef,
+                                                                   int* err)
 {
-    int i = blockIdx.x * blockDim.x + threadIdx.x;
-    int p = blockIdx.y >> 2, mu = blockIdx.y & 3;
+    int i = (blockIdx.x >> 3) * blockDim.x + threadIdx.x;
+    int p = (blockIdx.x >> 2) & 1, mu = blockIdx.x & 3;
     if (i >= g.Vh) return;
-    Walker x = link_coords(g, p, i);
+    const Coord c = eo_coords(g, p, i);
     M3 G = m3_zero();
 #pragma unroll 1
     for (int nu = 0; nu < 4; ++nu)
-        if (nu != mu) m3_acc(G, staple(V2, slot_of(nu, mu), V2, slot_of(mu, nu), g, x, mu, nu));
-    M3 Umu = ld_link(U, p, mu, i, g.Vh);
+        if (nu != mu) staple_acc(G, field(V2, slot_of(nu, mu), g), field(V2, slot_of(mu, nu), g), g, c, p, mu, nu);
     M3 out;
-    if (!smear_link(G, Umu, coef, out)) {
+    if (!smear_link(G, ld_link(U, p, mu, i, g.Vh), coef, out)) {
         atomicOr(err, DEV_ERR_DOMAIN);
-        out = Umu;
+        return;
     }
     st_link(U, p, mu, i, g.Vh, out);
 }
 
-dim3 link_grid(const Geom& g) { return dim3((g.Vh + kThreads - 1) / kThreads, 8); }
+// the parities, directions (and decorated directions) of a range of sites are
+// adjacent in the grid, so that their links meet in the L2 (at 24^4, where one
+// field is larger, a stout level 385 -> 288 us and a HEX pass 1955 -> 1639)
+unsigned link_grid(const Geom& g) { return 8u * ((g.Vh + kThreads - 1) / kThreads); }
+unsigned decorated_grid(const Geom& g) { return 24u * ((g.Vh + kThreads - 1) / kThreads); }
 
 // ---------------------------------------------------------------------------
 // Smeared-link force: the chain rule through stout levels (no counterpart in
@@ -201,8 +238,7 @@ __device__ __forceinline__ double xi1_stable(double w)
 // c1 = Tr Q^2 / 2); h_j as in expiq, dh_j/dw = w g_j, D = 9u^2 - w^2
 __device__ bool expiq_coeffs(const M3& Q, const M3& Q2, Z (&f)[3], Z (&d0)[3], Z (&d1)[3])
 {
-    M3 Q3 = m3_mul(Q2, Q);
-    double c0 = m3_tr(Q3).re / 3.0;
+    double c0 = m3_retr(Q2, Q) / 3.0;
     double c1 = 0.5 * m3_tr(Q2).re;
     if (c1 < 0.0) return false;
     if (c1 < 1e-12) {
@@ -288,33 +324,42 @@ __device__ __forceinline__ M3 m3_scale(const M3& a, Z s)
 // G = -2i V^dag F
 __global__ void __launch_bounds__(kThreads) sforce_top_kernel(Geom g, const void* V, const void* F, void* G)
 {
-    int i = blockIdx.x * blockDim.x + threadIdx.x;
-    int p = blockIdx.y >> 2, mu = blockIdx.y & 3;
+    int i = (blockIdx.x >> 3) * blockDim.x + threadIdx.x;
+    int p = (blockIdx.x >> 2) & 1, mu = blockIdx.x & 3;
     if (i >= g.Vh) return;
     st_link(G, p, mu, i, g.Vh, m3_scale(m3_adj_mul(ld_link(V, p, mu, i, g.Vh), ld_link(F, p, mu, i, g.Vh)), Z{0.0, -2.0}));
 }
 
-// per link of level U: W = U^dag K and Gn = G exp(iQ) - C^dag K
-__global__ void __launch_bounds__(kThreads) sforce_level_kernel(Geom g, const void* U, const void* G, void* W, void* Gn,
-                                                                double rho, int* err)
+// per link of level U: W = U^dag K and Gn = G exp(iQ) - C^dag K.  Q, Q^2, B and
+// two sums are live at once: 254 registers without spills, once the staples
+// wait in shared memory, U and G are read twice, and the traces of products
+// take no product
+__global__ void __launch_bounds__(kThreads, kForceOcc) sforce_level_kernel(Geom g, const void* U, const void* G, void* W,
+                                                                           void* Gn, double rho, int* err)
 {
-    int i = blockIdx.x * blockDim.x + threadIdx.x;
-    int p = blockIdx.y >> 2, mu = blockIdx.y & 3;
+    // the staples, needed again at the end, wait in shared memory
+    __shared__ double2 sC[9][kThreads];
+    int i = (blockIdx.x >> 3) * blockDim.x + threadIdx.x;
+    int p = (blockIdx.x >> 2) & 1, mu = blockIdx.x & 3;
     if (i >= g.Vh) return;
-    Walker x = link_coords(g, p, i);
-    M3 C = m3_zero();
+    M3 Q;
+    {
+        const Coord c = eo_coords(g, p, i);
+        M3 C = m3_zero();
 #pragma unroll 1
-    for (int nu = 0; nu < 4; ++nu)
-        if (nu != mu) m3_acc(C, staple(U, 0, U, 0, g, x, mu, nu));
-    const M3 u = ld_link(U, p, mu, i, g.Vh);
-    M3 om = m3_mul_adj(C, u), Q;
+        for (int nu = 0; nu < 4; ++nu)
+            if (nu != mu) staple_acc(C, (const double2*)U, (const double2*)U, g, c, p, mu, nu);
 #pragma unroll
-    for (int a = 0; a < 3; ++a)
+        for (int k = 0; k < 9; ++k) sC[k][threadIdx.x] = make_double2(C.e[k].re, C.e[k].im);
+        const M3 om = m3_mul_adj(C, ld_link(U, p, mu, i, g.Vh));
 #pragma unroll
-        for (int b = 0; b < 3; ++b) {
-            Z d = zd(om.e[a * 3 + b], cconj(om.e[b * 3 + a]));  // Q = -i rho TA(om)
-            Q.e[a * 3 + b] = {0.5 * rho * d.im, -0.5 * rho * d.re};
-        }
+        for (int a = 0; a < 3; ++a)
+#pragma unroll
+            for (int b = 0; b < 3; ++b) {
+                Z d = zd(om.e[a * 3 + b], cconj(om.e[b * 3 + a]));  // Q = -i rho TA(om)
+                Q.e[a * 3 + b] = {0.5 * rho * d.im, -0.5 * rho * d.re};
+            }
+    }
     m3_traceless(Q);
     const M3 Q2 = m3_mul(Q, Q);
     Z f[3], d0[3], d1[3];
@@ -322,61 +367,90 @@ __global__ void __launch_bounds__(kThreads) sforce_level_kernel(Geom g, const vo
         atomicOr(err, DEV_ERR_DOMAIN);
         return;
     }
-    M3 eq;
-#pragma unroll
-    for (int k = 0; k < 9; ++k) eq.e[k] = za(zm(f[1], Q.e[k]), zm(f[2], Q2.e[k]));
-    eq.e[0] = za(eq.e[0], f[0]);
-    eq.e[4] = za(eq.e[4], f[0]);
-    eq.e[8] = za(eq.e[8], f[0]);
-    const M3 Gl = ld_link(G, p, mu, i, g.Vh);
-    const M3 B = m3_mul(u, Gl);
-    const M3 BQ = m3_mul(B, Q), BQ2 = m3_mul(B, Q2), QB = m3_mul(Q, B);
-    const Z t0 = m3_tr(B), t1 = m3_tr(BQ), t2 = m3_tr(BQ2);
-    const Z b0 = za(za(zm(t0, d0[0]), zm(t1, d0[1])), zm(t2, d0[2]));
-    const Z b1 = za(za(zm(t0, d1[0]), zm(t1, d1[1])), zm(t2, d1[2]));
     M3 Lh;
+    {
+        const M3 B = m3_mul(ld_link(again((const double2*)U), p, mu, i, g.Vh), ld_link(G, p, mu, i, g.Vh));
+        // tr B, tr B Q, tr B Q^2
+        const Z t0 = m3_tr(B), t1 = m3_trmul(B, Q), t2 = m3_trmul(B, Q2);
+        const Z b0 = za(za(zm(t0, d0[0]), zm(t1, d0[1])), zm(t2, d0[2]));
+        const Z b1 = za(za(zm(t0, d1[0]), zm(t1, d1[1])), zm(t2, d1[2]));
+        M3 AQ = m3_mul(Q, B);  // Q B + B Q
+        m3_mul_to<true>(AQ, B, Q);
 #pragma unroll
-    for (int k = 0; k < 9; ++k)
-        Lh.e[k] = za(za(zm(b0, Q2.e[k]), zm(b1, Q.e[k])), za(zm(f[1], B.e[k]), zm(f[2], za(QB.e[k], BQ.e[k]))));
+        for (int k = 0; k < 9; ++k)
+            Lh.e[k] = za(za(zm(b0, Q2.e[k]), zm(b1, Q.e[k])), za(zm(f[1], B.e[k]), zm(f[2], AQ.e[k])));
+    }
+    M3 out;
+    {
+        M3 eq;
+#pragma unroll
+        for (int k = 0; k < 9; ++k) eq.e[k] = za(zm(f[1], Q.e[k]), zm(f[2], Q2.e[k]));
+        eq.e[0] = za(eq.e[0], f[0]);
+        eq.e[4] = za(eq.e[4], f[0]);
+        eq.e[8] = za(eq.e[8], f[0]);
+        out = m3_mul(ld_link(again((const double2*)G), p, mu, i, g.Vh), eq);
+    }
     const M3 K = m3_scale(m3_th(Lh), Z{0.0, -rho});
-    st_link(W, p, mu, i, g.Vh, m3_adj_mul(u, K));
-    M3 out = m3_mul(Gl, eq);
-    const M3 cK = m3_adj_mul(C, K);
-    m3_axpy(out, -1.0, cK);
+    st_link(W, p, mu, i, g.Vh, m3_adj_mul(ld_link(again((const double2*)U), p, mu, i, g.Vh), K));
+    M3 C;
+#pragma unroll
+    for (int k = 0; k < 9; ++k) {
+        const double2 v = sC[k][threadIdx.x];
+        C.e[k] = {v.x, v.y};
+    }
+    m3_axpy(out, -1.0, m3_adj_mul(C, K));
     st_link(Gn, p, mu, i, g.Vh, out);
 }
 
 // dS/dU of link (y, a): Gn + the staple terms Re Tr(W_l dC_l) of the links l
-// whose plaquette staples contain it (six positions, three directions each)
-__global__ void __launch_bounds__(kThreads) sforce_gather_kernel(Geom g, const void* U, const void* W, const void* Gn,
-                                                                 void* G)
+// whose plaquette staples contain it (six positions, three directions each).
+// The terms of a direction share links; held in registers from term to term
+// they spill, so each term reads its own (the L1 has them).  Level and gather:
+// 417 -> 277 us at 16^4, 2262 -> 1374 us at 24^4.  Six warps per 32 links, one
+// for each direction and side, were slower (339 and 1782 us).
+__global__ void __launch_bounds__(kThreads, kForceOcc) sforce_gather_kernel(Geom g, const void* Uf, const void* Wf,
+                                                                            const void* Gn, void* G)
 {
-    int i = blockIdx.x * blockDim.x + threadIdx.x;
-    int p = blockIdx.y >> 2, a = blockIdx.y & 3;
+    int i = (blockIdx.x >> 3) * blockDim.x + threadIdx.x;
+    int p = (blockIdx.x >> 2) & 1, a = blockIdx.x & 3;
     if (i >= g.Vh) return;
-    const Walker y = link_coords(g, p, i);
+    const Coord c = eo_coords(g, p, i);
+    const double2 *U = (const double2*)Uf, *W = (const double2*)Wf;
+    const int Vh = g.Vh, y = c.lex, ya = y + step_offset(g, c, a, 1), o = 1 - p;
     M3 out = ld_link(Gn, p, a, i, g.Vh);
 #pragma unroll 1
     for (int d = 0; d < 4; ++d) {
         if (d == a) continue;
-        Walker ya = y, yd = y, ymd = y;
-        walk(g, ya, a, +1);
-        walk(g, yd, d, +1);
-        walk(g, ymd, d, -1);
-        Walker ymda = ymd;
-        walk(g, ymda, a, +1);
+        const int yd = y + step_offset(g, c, d, 1), dm = step_offset(g, c, d, -1), ymd = y + dm, ymda = ya + dm;
+        M3 t;
         // U_nu(x) of an upper staple of (x = y, d)
-        m3_acc(out, m3_mul(m3_mul_adj(link_at(U, g, ya, d), link_at(U, g, yd, a)), link_at(W, g, y, d)));
+        t = m3_mul_adj(ld_at(U, Vh, o, d, ya), ld_at(U, Vh, o, a, yd));
+        m3_mul_to<true>(out, t, ld_at(W, Vh, p, d, y));
+        U = again(U);
+        W = again(W);
         // U_mu(x+nu) of an upper staple of (x = y - d, a)
-        m3_acc(out, m3_mul(m3_adj_mul(link_at(U, g, ymda, d), link_at(W, g, ymd, a)), link_at(U, g, ymd, d)));
+        t = m3_adj_mul(ld_at(U, Vh, p, d, ymda), ld_at(W, Vh, o, a, ymd));
+        m3_mul_to<true>(out, t, ld_at(U, Vh, o, d, ymd));
+        U = again(U);
+        W = again(W);
         // U_nu(x+mu) of an upper staple of (x = y - d, d): (W U_a(x) U_d(x+a))^dag
-        m3_acc(out, m3_adj(m3_mul(m3_mul(link_at(W, g, ymd, d), link_at(U, g, ymd, a)), link_at(U, g, ymda, d))));
+        t = m3_mul(ld_at(W, Vh, o, d, ymd), ld_at(U, Vh, o, a, ymd));
+        m3_mul_dag_acc(out, t, ld_at(U, Vh, p, d, ymda));
+        U = again(U);
+        W = again(W);
         // U_nu(x-nu) of a lower staple of (x = y + a, d): (U_d(y) U_a(y+d) W)^dag
-        m3_acc(out, m3_adj(m3_mul(m3_mul(link_at(U, g, y, d), link_at(U, g, yd, a)), link_at(W, g, ya, d))));
+        t = m3_mul(ld_at(U, Vh, p, d, y), ld_at(U, Vh, o, a, yd));
+        m3_mul_dag_acc(out, t, ld_at(W, Vh, o, d, ya));
+        U = again(U);
+        W = again(W);
         // U_mu(x-nu) of a lower staple of (x = y + d, a)
-        m3_acc(out, m3_mul_adj(m3_mul(link_at(U, g, ya, d), link_at(W, g, yd, a)), link_at(U, g, y, d)));
+        t = m3_mul(ld_at(U, Vh, o, d, ya), ld_at(W, Vh, o, a, yd));
+        m3_mul_adj_to<true>(out, t, ld_at(U, Vh, p, d, y));
+        U = again(U);
+        W = again(W);
         // U_nu(x-nu+mu) of a lower staple of (x = y - d + a, d)
-        m3_acc(out, m3_mul(m3_mul_adj(link_at(W, g, ymda, d), link_at(U, g, ymd, a)), link_at(U, g, ymd, d)));
+        t = m3_mul_adj(ld_at(W, Vh, p, d, ymda), ld_at(U, Vh, o, a, ymd));
+        m3_mul_to<true>(out, t, ld_at(U, Vh, o, d, ymd));
     }
     st_link(G, p, a, i, g.Vh, out);
 }
@@ -384,8 +458,8 @@ __global__ void __launch_bounds__(kThreads) sforce_gather_kernel(Geom g, const v
 // F = TH(i U G) / 2
 __global__ void __launch_bounds__(kThreads) sforce_bottom_kernel(Geom g, const void* U, const void* G, void* F)
 {
-    int i = blockIdx.x * blockDim.x + threadIdx.x;
-    int p = blockIdx.y >> 2, mu = blockIdx.y & 3;
+    int i = (blockIdx.x >> 3) * blockDim.x + threadIdx.x;
+    int p = (blockIdx.x >> 2) & 1, mu = blockIdx.x & 3;
     if (i >= g.Vh) return;
     M3 t = m3_th(m3_scale(m3_mul(ld_link(U, p, mu, i, g.Vh), ld_link(G, p, mu, i, g.Vh)), Z{0.0, 0.5}));
     st_link(F, p, mu, i, g.Vh, t);
@@ -393,13 +467,13 @@ __global__ void __launch_bounds__(kThreads) sforce_bottom_kernel(Geom g, const v
 
 }  // namespace
 
-// n stout levels; U is updated in place, tmp is one link field of scratch
+// n stout levels; U is updated, tmp is one link field of scratch.  The levels
+// alternate between the two; an odd count takes one copy back.
 cudaError_t launch_stout(const Geom& g, void* U, void* tmp, double rho, int n, int* err, cudaStream_t s)
 {
-    for (int k = 0; k < n; ++k) {
-        stout_kernel<<<link_grid(g), kThreads, 0, s>>>(g, U, tmp, rho, err);
-        cudaMemcpyAsync(U, tmp, (size_t)g.V * 4 * 9 * 16, cudaMemcpyDeviceToDevice, s);
-    }
+    for (int k = 0; k < n; ++k)
+        stout_kernel<<<link_grid(g), kThreads, 0, s>>>(g, k & 1 ? tmp : U, k & 1 ? U : tmp, rho, err);
+    if (n & 1) cudaMemcpyAsync(U, tmp, (size_t)g.V * 4 * 9 * 16, cudaMemcpyDeviceToDevice, s);
     return cudaGetLastError();
 }
 
@@ -499,8 +573,8 @@ cudaError_t launch_hex(const Geom& g, void* U, void* scratch, double a1, double 
     char* V1 = (char*)scratch;
     char* V2 = V1 + (size_t)3 * g.V * 4 * 9 * 16;
     for (int k = 0; k < n; ++k) {
-        hex1_kernel<<<link_grid(g), kThreads, 0, s>>>(g, U, V1, 0.5 * a3, err);
-        hex2_kernel<<<link_grid(g), kThreads, 0, s>>>(g, U, V1, V2, 0.5 * a2, err);
+        hex1_kernel<<<decorated_grid(g), kThreads, 0, s>>>(g, U, V1, 0.5 * a3, err);
+        hex2_kernel<<<decorated_grid(g), kThreads, 0, s>>>(g, U, V1, V2, 0.5 * a2, err);
         hex3_kernel<<<link_grid(g), kThreads, 0, s>>>(g, U, V2, 0.5 * a1, err);
     }
     return cudaGetLastError();

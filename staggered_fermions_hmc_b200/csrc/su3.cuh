@@ -122,6 +122,36 @@ __device__ __forceinline__ M3 m3_adj_mul(const M3& a, const M3& b)
     return o;
 }
 
+// o += (a b)^dag
+__device__ __forceinline__ void m3_mul_dag_acc(M3& o, const M3& a, const M3& b)
+{
+#pragma unroll
+    for (int i = 0; i < 3; ++i)
+#pragma unroll
+        for (int j = 0; j < 3; ++j) {
+            Cx<double>& s = o.e[i * 3 + j];  // += conj(sum_k a_jk b_ki)
+#pragma unroll
+            for (int k = 0; k < 3; ++k) {
+                const Cx<double> x = a.e[j * 3 + k], y = b.e[k * 3 + i];
+                s.re = fma(x.re, y.re, s.re);
+                s.im = fma(-x.re, y.im, s.im);
+                s.re = fma(-x.im, y.im, s.re);
+                s.im = fma(-x.im, y.re, s.im);
+            }
+        }
+}
+
+// tr(a b)
+__device__ __forceinline__ Cx<double> m3_trmul(const M3& a, const M3& b)
+{
+    Cx<double> s = {0.0, 0.0};
+#pragma unroll
+    for (int i = 0; i < 3; ++i)
+#pragma unroll
+        for (int k = 0; k < 3; ++k) cfma<false>(s, a.e[i * 3 + k], b.e[k * 3 + i]);
+    return s;
+}
+
 // Re tr(a b), Re tr(a b^dag)
 __device__ __forceinline__ double m3_retr(const M3& a, const M3& b)
 {
@@ -216,8 +246,7 @@ __device__ __forceinline__ double sinc_stable(double x)
 __device__ __forceinline__ bool expiq(const M3& Q, M3& out)
 {
     M3 Q2 = m3_mul(Q, Q);
-    M3 Q3 = m3_mul(Q2, Q);
-    Cx<double> t3 = m3_tr(Q3);
+    Cx<double> t3 = m3_trmul(Q2, Q);
     if (fabs(t3.im) > 1e-10) return false;
     double c0 = t3.re / 3.0;
     double c1 = 0.5 * m3_tr(Q2).re;

@@ -7,6 +7,27 @@
 
 namespace sfh {
 
+// coordinate and extent of a runtime direction, without indexing an array
+__device__ __forceinline__ int coord_of(const Coord& c, int mu)
+{
+    return mu == 0 ? c.x[0] : (mu == 1 ? c.x[1] : (mu == 2 ? c.x[2] : c.x[3]));
+}
+
+__device__ __forceinline__ int extent_of(const Geom& g, int mu)
+{
+    return mu == 0 ? g.L[0] : (mu == 1 ? g.L[1] : (mu == 2 ? g.L[2] : g.L[3]));
+}
+
+// lexicographic offset of x + k mu, |k| <= 2 <= L (periodic)
+__device__ __forceinline__ int step_offset(const Geom& g, const Coord& c, int mu, int k)
+{
+    const int L = extent_of(g, mu), x = coord_of(c, mu);
+    int y = x + k;
+    if (y < 0) y += L;
+    if (y >= L) y -= L;
+    return (y - x) * lex_stride(g, mu);
+}
+
 struct Walker {
     int x[4];
 };

@@ -537,3 +537,29 @@ def test_heatbath_at_unequal_extents(sfh, orc, dims):
     lat.heatbath_update(n_sweeps=2, seed=29, sweep0=1)
     assert rel(lat.download_gauge(), orc.heatbath(dims, 4.2, U, seed=29, nsweeps=2, sweep0=1)) < 1e-12
     lat.close()
+
+
+@pytest.mark.parametrize("dims", [(2, 2, 2, 2), (2, 6, 4, 2), (6, 2, 2, 10), (4, 6, 10, 6)])
+def test_smearing_kernels_at_odd_sizes(sfh, orc, dims):
+    """Stout (odd and even level counts end in different buffers), HEX and the
+    chain-rule force where the last block of a direction is not full and both
+    neighbours of a site are the same (extent 2), with the tolerances of the
+    tests above."""
+    U = orc.random_gauge(dims, 0.3, 211)
+    lat = sfh.Lattice(dims, 0.3, 4.2)
+    for n in (1, 2, 3):
+        lat.upload_gauge(U)
+        lat.smear_stout(0.125, n)
+        assert rel(lat.download_gauge(), orc.stout(dims, 0.125, n, U)) < 1e-12
+    lat.upload_gauge(U)
+    lat.Apply_HEX_smearing()
+    assert rel(lat.download_gauge(), orc.hex_smear(dims, U)) < 1e-12
+    lat.upload_gauge(U)
+    lat.set_fermion_smearing(0.125, 2)
+    phi = orc.random_spinor(dims, 212)
+    F, X = lat.smeared_fermion_force(phi, tol=1e-13)
+    Vs = orc.stout(dims, 0.125, 2, U)
+    Xo = orc.cg(dims, 0.3, Vs, phi, 1e-13)[0]
+    Yo = orc.dirac(dims, 0.3, Vs, Xo, dagger=True)
+    assert rel(F, orc.stout_force(dims, 0.125, 2, U, orc.fermion_force(dims, Vs, Xo, Yo))) < 1e-10
+    lat.close()
