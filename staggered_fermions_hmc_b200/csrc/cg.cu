@@ -158,6 +158,22 @@ __device__ __forceinline__ ItemRange item_range(const CgArgs& a, const CgSys& S,
     return r;
 }
 
+// The kernels of an iteration are chained by programmatic dependencies
+// (ensure_graph): a kernel's blocks may start, as SMs drain, once all blocks
+// of the kernel before it have started.  Up to here a block reads only what
+// does not change during a solve (its work item, system and vector table);
+// the wait ends when the kernel before is complete and its writes are
+// visible.  Its own successor is let go after the wait, so that no more than
+// two kernels of the chain are in flight.  Launched without such a
+// dependency, both instructions do nothing.  Measured, whole solves: six small
+// FP64 systems (36 us per iteration) 22.7 -> 20.9 ms, FP64 16^4 with 4 RHS
+// 17.5 -> 17.0, FP32 24^4 21.6 -> 20.7, FP16 32^3 64 111.8 -> 109.7.
+__device__ __forceinline__ void pdl_begin()
+{
+    asm volatile("griddepcontrol.wait;" ::: "memory");
+    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+}
+
 // Link staging: every thread copies the 8 links of its site (4 forward at
 // the site, 4 backward at its neighbours) into its own columns of shared
 // memory with asynchronous copies, [direction][element][thread], so that all
@@ -617,6 +633,7 @@ __device__ __forceinline__ void hop1_item(const CgArgs& a, const int2 it, int cu
         pp[l] = l < cnt ? rhs_ptr(a, S.rhs0 + base + l, F_P) : nullptr;
         tout[l] = l < cnt ? rhs_ptr(a, S.rhs0 + base + l, F_T) : nullptr;
     }
+    pdl_begin();
     gather_pass<NB>(a, S, base, q, true, cur, false, P);
     if (!(P.anyA || (ru_here && P.anyR))) return;
     const void* pin[NB];
@@ -693,6 +710,7 @@ __global__ void __launch_bounds__(kTile, (HopOcc<GP, SP, NB, false, RUI>::v))
 {
     if constexpr (DYN) {
         __shared__ int s_next;
+        pdl_begin();
         for (;;) {
             if (threadIdx.x == 0) s_next = atomicAdd(a.qctr + 2 * cur + 0, 1);
             __syncthreads();
@@ -727,6 +745,7 @@ __device__ __forceinline__ void hop2_item(const CgArgs& a, const int2 it, int cu
     // the reliable-update residuals are computed here too: measured faster
     // than a kernel of their own, and the compiler keeps the FP64 hop's
     // registers better with them here
+    pdl_begin();
     gather_pass<NB>(a, S, item_rhs(it), q, false, cur, false, P);
     if (!(P.anyA || (RUI && P.anyR))) return;  // uniform across the block
     bool part[NB], on[NB];
@@ -836,6 +855,7 @@ __global__ void __launch_bounds__(kTile, (HopOcc<GP, SP, NB, true, RUI>::v))
 {
     if constexpr (DYN) {
         __shared__ int s_next;
+        pdl_begin();
         for (;;) {
             if (threadIdx.x == 0) s_next = atomicAdd(a.qctr + 2 * cur + 1, 1);
             __syncthreads();
@@ -857,15 +877,6 @@ __device__ __forceinline__ void update_body(const CgArgs& a, int2 it, int cur, C
     typedef typename SpinorFmt<SP>::R RS;
     constexpr int XP = XFmt<SP>::v;
     typedef typename SpinorFmt<XP>::R RX;
-    // this iteration's reliable-update list was read by the kernels before
-    // this one: empty it for the iteration after next
-    if (a.ru_list && blockIdx.x == 0 && threadIdx.x == 0) a.ru_list[cur * (a.nlanes + 1)] = 0;
-    // this iteration's hop kernels have taken their work items: their
-    // counters start from zero again two iterations on
-    if (a.qctr && blockIdx.x == 0 && threadIdx.x == 0) {
-        a.qctr[2 * cur] = 0;
-        a.qctr[2 * cur + 1] = 0;
-    }
     stage_item_sys(a, it, s_sys);
     const CgSys& S = *s_sys;
     const ItemRange ir = item_range(a, S, it.x);
@@ -875,6 +886,16 @@ __device__ __forceinline__ void update_body(const CgArgs& a, int2 it, int cur, C
     void* rp = rhs_ptr(a, rid, F_R);
     void* xp = rhs_ptr(a, rid, F_XLO);
     const void* vp = rhs_ptr(a, rid, F_V);
+    if constexpr (!COH) pdl_begin();
+    // this iteration's reliable-update list was read by the kernels before
+    // this one: empty it for the iteration after next
+    if (a.ru_list && blockIdx.x == 0 && threadIdx.x == 0) a.ru_list[cur * (a.nlanes + 1)] = 0;
+    // this iteration's hop kernels have taken their work items: their
+    // counters start from zero again two iterations on
+    if (a.qctr && blockIdx.x == 0 && threadIdx.x == 0) {
+        a.qctr[2 * cur] = 0;
+        a.qctr[2 * cur + 1] = 0;
+    }
     CgLane* L = a.lanes + lane_of(S, item_rhs(it), q, false);
     const int mode = ld_int(&L->mode[cur]);
     if (mode != LM_ACTIVE && mode != LM_RESTART && mode != LM_LAST) return;
@@ -1250,6 +1271,7 @@ template <int SP>
 __global__ void __launch_bounds__(kTile, kListBlocksPerSm) cg_ru1_list(CgArgs a, const int2* __restrict__, int cur)
 {
     __shared__ CgSys s_sys;
+    pdl_begin();
     ru1_list_body<SP, false>(a, cur, blockIdx.x, gridDim.x, &s_sys);
 }
 
@@ -1259,6 +1281,7 @@ __global__ void __launch_bounds__(kTile, kListBlocksPerSm) cg_ru2_list(CgArgs a,
     __shared__ CgSys s_sys;
     __shared__ double s_bs[32];
     __shared__ unsigned s_mask;
+    pdl_begin();
     ru2_list_body<SP, false>(a, cur, blockIdx.x, gridDim.x, &s_sys, s_bs, &s_mask);
 }
 
@@ -1268,6 +1291,7 @@ __global__ void __launch_bounds__(kTile, (SysOcc<GP, false>::v)) cg_hop1_sys(CgA
 {
     extern __shared__ __align__(16) unsigned char s_dyn[];
     __shared__ CgSys s_sys;
+    pdl_begin();
     hop1_sys_body<GP, SP, NB, false>(a, items[blockIdx.x].x, cur, &s_sys, s_dyn);
 }
 
@@ -1280,6 +1304,7 @@ __global__ void __launch_bounds__(kTile, (SysOcc<GP, true>::v)) cg_hop2_sys(CgAr
     __shared__ float s_red[NB * kSums][kTile];
     __shared__ double s_tot[NB * kSums];
     __shared__ unsigned s_mask;
+    pdl_begin();
     hop2_sys_body<GP, SP, NB, false>(a, items[blockIdx.x].x, cur, &s_sys, s_dyn, s_red, s_tot, &s_mask);
 }
 
@@ -1891,8 +1916,14 @@ static cudaError_t ensure_graph(CgWorkspace& w, const CgKernels& k, CgArgs a, do
             void* args[] = {&a, (void*)&items[j], &cur};
             p.kernelParams = args;
             cudaGraphNode_t node;
-            e = cudaGraphAddKernelNode(&node, w.graph, prev ? &prev : nullptr, prev ? 1 : 0, &p);
-            if (e != cudaSuccess) return e;
+            if ((e = cudaGraphAddKernelNode(&node, w.graph, nullptr, 0, &p)) != cudaSuccess) return e;
+            if (prev) {  // a programmatic dependency: pdl_begin
+                cudaGraphEdgeData edge;
+                std::memset(&edge, 0, sizeof(edge));
+                edge.from_port = cudaGraphKernelNodePortProgrammatic;
+                edge.type = cudaGraphDependencyTypeProgrammatic;
+                if ((e = cudaGraphAddDependencies_v2(w.graph, &prev, &node, &edge, 1)) != cudaSuccess) return e;
+            }
             prev = node;
         }
     }

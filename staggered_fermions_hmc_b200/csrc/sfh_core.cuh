@@ -210,14 +210,15 @@ enum GaugePrec { GP_F64_18 = 0, GP_F32_12 = 1, GP_F16_12 = 2, GP_F32_18 = 3, GP_
 
 template <int SP> struct SpinorFmt;
 
-// load of a vector word: through the read-only data cache (COH false; data
-// not written while the kernel runs) or through L2 only (COH true: data other
-// blocks of the same persistent kernel write between its phases)
+// load of a vector word: through the L1 (COH false; not as read-only data,
+// since a kernel launched early by pdl_begin is there while its input is
+// written) or through L2 only (COH true: data other blocks of the same
+// persistent kernel write between its phases)
 template <bool COH, typename T>
 __device__ __forceinline__ T ld_vec(const T* p)
 {
     if constexpr (COH) return __ldcg(p);
-    else return __ldg(p);
+    else return *p;
 }
 
 template <> struct SpinorFmt<SP_F64> {
