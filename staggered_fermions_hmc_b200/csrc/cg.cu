@@ -370,19 +370,12 @@ __device__ __forceinline__ void lane_stop(const CgArgs& a, CgLane* L, int cur, i
     atomicSub(a.n_active, 1);
 }
 
-// Advance one lane's FP64 scalars from the summed partials of hop2 (warp 0).
+// Advance one lane's FP64 scalars from the summed partials of hop2 (one thread).
 // The update of this iteration (x += alpha p, r -= alpha v, p = r + beta p)
 // still runs for an ACTIVE lane; the decision applies from the next one.
-__device__ __forceinline__ void finish_lane(const CgArgs& a, const CgSys& S, int lane, int mode, int cur)
+__device__ __forceinline__ void advance_lane(const CgArgs& a, int lane, int mode, int cur, const double (&s)[kSums])
 {
     CgLane* L = a.lanes + lane;
-    const int nslot = 2 * S.ntq;
-    const int nsq = item_groups(a, S);
-    const double* base = a.partial + L->poff + (S.both ? 0 : L->parity * nsq);
-    const int n = S.both ? 2 * nsq : nsq;
-    double s[kSums];
-    warp_sum_slots_n<kSums>(base, nslot, n, s);
-    if (threadIdx.x != 0) return;
     const int nxt = cur ^ 1;
     if (mode == LM_ACTIVE || mode == LM_RESTART) {
         const double rr = s[3], pAp = s[0];
@@ -447,6 +440,66 @@ __device__ __forceinline__ void finish_lane(const CgArgs& a, const CgSys& S, int
             L->rmax = sqrt(rt);
             L->mode[nxt] = restart ? LM_RESTART : LM_ACTIVE;
         }
+    }
+}
+
+// advance_lane on the sums of the lane's slots (warp 0)
+__device__ __forceinline__ void finish_lane(const CgArgs& a, const CgSys& S, int lane, int mode, int cur)
+{
+    CgLane* L = a.lanes + lane;
+    const int nslot = 2 * S.ntq;
+    const int nsq = item_groups(a, S);
+    const double* base = a.partial + L->poff + (S.both ? 0 : L->parity * nsq);
+    const int n = S.both ? 2 * nsq : nsq;
+    double s[kSums];
+    warp_sum_slots_n<kSums>(base, nslot, n, s);
+    if (threadIdx.x == 0) advance_lane(a, lane, mode, cur, s);
+}
+
+// Advance every active lane, a block per lane: what the last block of the
+// second hop does for a lane (finish_lane), done by the kernel after it.  A
+// block of the hop then leaves once its partial sums are stored; the fence,
+// ticket and wait of every block took 4 to 5 us in which its successor could
+// not start (FP16 32^3 64, one tile an item: hop 184 -> 137 us a launch, four
+// tiles 141 -> 131; the uneven batch 118 -> 110; this part adds 3 us to the
+// kernel that does it).  The slots are added in the same order, 256 of each
+// sum at a time through shared memory.
+__device__ __forceinline__ void finish_lanes(const CgArgs& a, int cur, int blk, int nblk, double (&s_slots)[kSums][kTile],
+                                             double* s_tot)
+{
+    const int t = threadIdx.x, lane32 = t & 31, warp = t >> 5;
+    for (int lane = nblk - 1 - blk; lane < a.nlanes; lane += nblk) {
+        CgLane* L = a.lanes + lane;
+        const int mode = ld_int(&L->mode[cur]);
+        if (mode != LM_ACTIVE && mode != LM_RESTART) continue;  // uniform in the block
+        const CgSys& S = a.sys[L->sys];
+        const int nslot = 2 * S.ntq, nsq = item_groups(a, S);
+        const double* base = a.partial + L->poff + L->parity * nsq;
+        double v[kSums], sum = 0.0;
+#pragma unroll
+        for (int f = 0; f < kSums; ++f) v[f] = t < nsq ? __ldcg(base + (size_t)f * nslot + t) : 0.0;
+        for (int k0 = 0; k0 < nsq; k0 += kTile) {
+#pragma unroll
+            for (int f = 0; f < kSums; ++f) s_slots[f][t] = v[f];
+            __syncthreads();
+            const int k = k0 + kTile + t;
+#pragma unroll
+            for (int f = 0; f < kSums; ++f) v[f] = k < nsq ? __ldcg(base + (size_t)f * nslot + k) : 0.0;
+            if (warp < kSums)
+                for (int u = lane32; u < min(kTile, nsq - k0); u += 32) sum += s_slots[warp][u];
+            __syncthreads();
+        }
+        if (warp < kSums) {
+#pragma unroll
+            for (int o = 16; o > 0; o >>= 1) sum += __shfl_xor_sync(0xffffffffu, sum, o);
+            if (lane32 == 0) s_tot[warp] = sum;
+        }
+        __syncthreads();
+        if (t == 0) {
+            const double s[kSums] = {s_tot[0], s_tot[1], s_tot[2], s_tot[3]};
+            advance_lane(a, lane, mode, cur, s);
+        }
+        __syncthreads();
     }
 }
 
@@ -736,7 +789,7 @@ __device__ __forceinline__ void hop2_item(const CgArgs& a, const int2 it, int cu
     constexpr int XP = XFmt<SP>::v;
     __shared__ CgSys s_sys;
     __shared__ double smem[32 * NB * kSums];
-    __shared__ unsigned s_mask;
+    [[maybe_unused]] __shared__ unsigned s_mask;
     stage_item_sys(a, it, &s_sys);
     const CgSys& S = s_sys;
     const ItemRange ir = item_range(a, S, it.x);
@@ -835,13 +888,27 @@ __device__ __forceinline__ void hop2_item(const CgArgs& a, const int2 it, int cu
                     sums[l * kSums + 3] += ru_hop2<SP, XP>(a.rhs, S, c, q, ti.i, P.rid[l], P.m2[l]);
         }
     }
-    block_sum<NB * kSums>(sums, smem);
-    const unsigned nsq = (unsigned)item_groups(a, S);
-    unsigned mask = arrive_sums<NB>(a, S, P, part, sums, ir.slot, S.both ? 2u * nsq : nsq, &s_mask);
-    if (mask && threadIdx.x < 32) {
+    if constexpr (!RUI) {  // finish_lanes, in cg_ru2_list
+        double* dst[NB];
+        if (threadIdx.x == 0)
 #pragma unroll
-        for (int l = 0; l < NB; ++l)
-            if (mask & (1u << l)) finish_lane(a, S, P.lane[l], P.mode[l], cur);
+            for (int l = 0; l < NB; ++l) dst[l] = a.partial + __ldg(&a.lanes[P.lane[l]].poff) + ir.slot;
+        block_sum<NB * kSums>(sums, smem);
+        if (threadIdx.x == 0)
+#pragma unroll
+            for (int l = 0; l < NB; ++l)
+                if (part[l])
+#pragma unroll
+                    for (int f = 0; f < kSums; ++f) __stcg(dst[l] + f * 2 * S.ntq, sums[l * kSums + f]);
+    } else {
+        block_sum<NB * kSums>(sums, smem);
+        const unsigned nsq = (unsigned)item_groups(a, S);
+        unsigned mask = arrive_sums<NB>(a, S, P, part, sums, ir.slot, S.both ? 2u * nsq : nsq, &s_mask);
+        if (mask && threadIdx.x < 32) {
+#pragma unroll
+            for (int l = 0; l < NB; ++l)
+                if (mask & (1u << l)) finish_lane(a, S, P.lane[l], P.mode[l], cur);
+        }
     }
 }
 
@@ -1281,7 +1348,9 @@ __global__ void __launch_bounds__(kTile, kListBlocksPerSm) cg_ru2_list(CgArgs a,
     __shared__ CgSys s_sys;
     __shared__ double s_bs[32];
     __shared__ unsigned s_mask;
+    __shared__ double s_slots[kSums][kTile];
     pdl_begin();
+    if (a.finish_late) finish_lanes(a, cur, blockIdx.x, gridDim.x, s_slots, s_bs);
     ru2_list_body<SP, false>(a, cur, blockIdx.x, gridDim.x, &s_sys, s_bs, &s_mask);
 }
 
@@ -1870,6 +1939,7 @@ static CgArgs make_args(const CgWorkspace& w, double tol, int maxit, double delt
     a.maxloop = a.mixed ? 2 * maxit + 64 : maxit + 1;
     a.tpi = tpi;
     a.ru_list = nullptr;
+    a.finish_late = 0;
     a.nst_words = 0;
     a.err = nullptr;
     a.qctr = nullptr;
@@ -2094,22 +2164,33 @@ static cudaError_t flow_solve(CgWorkspace& w, const CgArgs& a, cudaStream_t stre
 // (widths, tiles per work item, staging; 0: as below).  It never changes the
 // mixed precisions' results.
 //
-// Several RHS or systems: groups of two, in FP16 of four in the first hop; from
+// Several RHS or systems: groups of two, in FP16 of four in the first hop, in
+// FP32 of one where no system has more than two RHS (24^4 with 2 RHS 47.8 ->
+// 38.9 ms, 24^3 48 43.7 -> 38.5; with 4 to 8 RHS the widths are equal); from
 // 400000 sites x RHS on the reliable updates in the lane-list kernels (two more
 // launches; FP16 and FP32-12: the BF16 hop gains less from their registers, the
 // FP32 18-real one is a third slower without them inline).  Against groups of
 // eight and four with inline updates, ms: 20 uneven systems, 94 RHS, FP16 225 ->
-// 192, FP32 277 -> 230, BF16 262 -> 232; 16^4 with 8 RHS FP16 28.6 -> 23.6; below
+// 183, FP32 277 -> 230, BF16 262 -> 232; 16^4 with 8 RHS FP16 28.6 -> 23.6; below
 // the line, 20^4 with 2 RHS, the lane lists would take 21.3 for 20.2.
 //
-// One RHS: the tiles per item and the staging of least cost, counted in tile
-// times of an SM: B = ceil(items / SMs) blocks of `tiles` tiles each, four for
-// every wave of resident blocks (launch, descriptors, partial last wave) and
+// FP64: groups of two read a link once for both, but a block takes 1.6 times as
+// long as one of a single RHS, which tells where there are few waves: by the
+// waves of resident blocks (six systems of up to 10^4, 22 RHS, 20.9 -> 19.4 ms;
+// 16^4 with 4 RHS stays at two, 17.0 against 20.9).
+//
+// One RHS, 16-bit storage: from 2000 tiles on the lane lists and two tiles an
+// item, from 6000 on four.  ms for two tiles with inline updates, lane lists
+// with two, with four: FP16 24^3 32 (1728 tiles) 13.6, 14.1, 15.3; 28^4 20.1, 18.6,
+// 19.0; 32^4 32.9, 30.1, 32.5; 32^3 64 61.6, 58.2, 56.9; BF16 24^3 32 14.5, 14.3,
+// 15.9; 28^4 21.3, 20.1, 22.3; 32^4 38.2, 32.6, 32.6; 32^3 64 74.9, 61.5, 60.4.
+//
+// One RHS, FP32: the tiles per item and the staging of least cost, counted in
+// tile times of an SM: B = ceil(items / SMs) blocks of `tiles` tiles each, four
+// for every wave of resident blocks (launch, descriptors, partial last wave) and
 // three for the two more kernels of the lane lists.  Against two tiles and
-// inline updates, m 0.2, ms: FP32 24^3 32 17.3 -> 14.4, 24^4 13.3 -> 12.4 and
-// 32^3 64 77.9 -> 71.6; FP16 28^4 20.4 -> 19.3, 32^4 (m 0.1) 61.0 -> 51.1; BF16
-// 32^3 64 76.4 -> 65.5.  On smaller lattices the 16-bit storages gained nothing
-// (18 22 26 30: FP16 10.9 against 11.3), nor did FP64 and FP32 18-real anywhere.
+// inline updates, ms: 24^3 32 16.2 -> 13.6, 32^4 39.7 -> 30.9, 32^3 64 76.3 ->
+// 69.3.  FP32 18-real gained nothing anywhere.
 struct AutoSchedule {
     int nb1 = 0, nb2 = 0, tpi = 0, stage = 0;
 };
@@ -2117,7 +2198,17 @@ struct AutoSchedule {
 static AutoSchedule auto_schedule(const CgWorkspace& w)
 {
     AutoSchedule s;
-    if (w.prec == SFH_PREC_F64) return s;
+    if (w.prec == SFH_PREC_F64) {
+        // waves of resident blocks of groups of two (1.6 times as long) and of one
+        long b1 = 0, b2 = 0;
+        for (const CgSys& S : w.sys) {
+            b1 += 2L * S.ntq * S.nrhs;
+            b2 += 2L * S.ntq * ((S.nrhs + 1) / 2);
+        }
+        const long slots = (long)HopOcc<GP_F64_18, SP_F64, 2, true>::v * std::max(1, w.num_sms);
+        if (5 * ((b1 + slots - 1) / slots) < 8 * ((b2 + slots - 1) / slots)) s.nb1 = s.nb2 = 1;
+        return s;
+    }
     const bool f16 = w.prec == SFH_PREC_F16, f32 = w.prec == SFH_PREC_F32;
     if (w.nlanes > 2) {
         if (w.auto_nb > 0) return s;  // a pair of masses keeps its own widths
@@ -2127,21 +2218,24 @@ static AutoSchedule auto_schedule(const CgWorkspace& w)
             work += (long)S.g.V * S.nrhs;
             most = std::max(most, S.nrhs);
         }
-        s.nb1 = default_nb(most, f16 ? 4 : 2);
-        s.nb2 = default_nb(most, 2);
+        s.nb1 = default_nb(most, f16 ? 4 : (f32 && most <= 2 ? 1 : 2));
+        s.nb2 = default_nb(most, f32 && most <= 2 ? 1 : 2);
         s.stage = (f16 || f32) && work >= 400000 ? 4 : 0;
         return s;
     }
     if (w.prec == SFH_PREC_F32_18) return s;
     const int sms = std::max(1, w.num_sms), tiles = 2 * w.sys[0].ntq;
-    if (!f32 && tiles < (f16 ? 2000 : 4000)) return s;
+    if (!f32) {
+        if (tiles < 2000) return s;
+        s.tpi = tiles < 6000 ? 2 : 4;
+        s.stage = 4;
+        return s;
+    }
     int best = 1 << 30;
     for (int stage : {0, 4})
-        for (int tpi : {1, 2, 4, 8, 16}) {
-            const int occ = stage == 0 ? (f16 ? HopOcc<GP_F16_12, SP_F16, 1, true, true>::v
-                                              : HopOcc<GP_F32_12, SP_F32, 1, true, true>::v)
-                                       : (f16 ? HopOcc<GP_F16_12, SP_F16, 1, true, false>::v
-                                              : HopOcc<GP_F32_12, SP_F32, 1, true, false>::v);
+        for (int tpi : {1, 2, 4, 8}) {
+            const int occ = stage == 0 ? HopOcc<GP_F32_12, SP_F32, 1, true, true>::v
+                                       : HopOcc<GP_F32_12, SP_F32, 1, true, false>::v;
             const int items = 2 * ((tiles / 2 + tpi - 1) / tpi), B = (items + sms - 1) / sms;
             // a block alone on its SM does not keep it busy
             const int cost = std::max(B, 2) * tpi + 4 * ((B + occ - 1) / occ) + (stage ? 3 : 0);
@@ -2246,6 +2340,7 @@ static cudaError_t workspace_solve(CgWorkspace& w, double tol, int maxit, double
     }
     if (k.ru1 || k.pers) {  // reliable updates by lane list: both lists start empty
         a.ru_list = w.d_rulist;
+        a.finish_late = k.ru2 && !k.sys;
         if ((e = cudaMemsetAsync(w.d_rulist, 0, sizeof(int) * 2 * (w.nlanes + 1), stream)) != cudaSuccess) return e;
     }
     k.init<<<w.ntiles, kTile, 0, stream>>>(a);

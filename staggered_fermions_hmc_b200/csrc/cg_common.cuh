@@ -62,6 +62,9 @@ struct CgArgs {
     // lanes due for a reliable update, per iteration parity: [2][1 + nlanes],
     // a count then lane ids (null: the hop kernels do the reliable updates)
     int* ru_list;
+    // the second reliable-update kernel completes the lanes' sums, not the
+    // second hop's last block (finish_lanes)
+    int finish_late;
     // neighbour staging (schedule 6): shared-memory words of one RHS's staged
     // range per buffer (kTile + the batch's largest Lt), and the device error
     // word a staging wait that gives up sets DEV_ERR_TIMEOUT in (null: unused)

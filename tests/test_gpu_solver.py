@@ -639,3 +639,52 @@ def test_dataflow_solve_full_lattice_masses_and_stops(sfh, orc):
             B.solve(tol=tol, max_iter=5)
         assert e.value.status == sfh.SFH_ERR_NOCONV
         B.close()
+
+
+@pytest.mark.parametrize("precision", ["f32", "f16", "bf16", "f32_18"])
+@pytest.mark.parametrize("dims,nrhs", [((2, 2, 2, 4), 3), ((4, 6, 8, 10), 2), ((16, 16, 16, 36), 1)])
+def test_lane_sums_completed_after_the_second_hop(sfh, precision, dims, nrhs):
+    """With the lane-list kernels the lanes' sums are completed by the kernel
+    after the second hop, by one block per lane, 256 slots at a time (the
+    last lattice has 288 per lane, the first one): solutions, iterations and
+    stops at max_iter equal those of the hop's own last block bit for bit."""
+    out = []
+    for schedule in ((1, 1, 0), (1, 1, 4), (2, 1, 4), (1, 1, 5), (1, 1, 6), (1, 1, 7)):
+        B = sfh.Batch([(dims, 0.2, nrhs), ((4, 4, 4, 4), 0.1, 1)], precision=precision)
+        B.set_schedule(*schedule)
+        for k, n in ((0, nrhs), (1, 1)):
+            B.random_gauge(k, 0.5, 31 + k)
+            for j in range(n):
+                B.random_rhs(k, j, 41 + 10 * k + j)
+        got = []
+        for max_iter in (7, 20000):
+            B.solve(tol=1e-10, max_iter=max_iter, check=max_iter > 7)
+            for k, n in ((0, nrhs), (1, 1)):
+                for j in range(n):
+                    got += [B.solution(k, j), B.info(k, j)["iters"], B.info(k, j)["status"]]
+        out.append(got)
+        B.close()
+    for o in out[1:]:
+        assert all(np.array_equal(a, b) for a, b in zip(o, out[0]))
+
+
+def test_fp64_group_widths_agree(sfh):
+    """FP64 systems solved by the per-phase kernels without a schedule take
+    groups of one or two right-hand sides by size.  The widths' solutions are
+    the same bit for bit; without a schedule (the dataflow kernel, or one of
+    the widths) the true residual is below 1.5 tol."""
+    tol = 1e-10
+    for systems in ([((10, 10, 10, 10), 0.2, n) for n in (2, 4, 8)], [((16, 16, 16, 16), 0.2, 4)]):
+        out = []
+        for schedule in ((1, 1, 0), (2, 1, 0), (0, 0, 0)):
+            B = sfh.Batch(systems, precision="f64")
+            B.set_schedule(*schedule)
+            for k, (d, m, n) in enumerate(systems):
+                B.random_gauge(k, 0.4, 51 + k)
+                for j in range(n):
+                    B.random_rhs(k, j, 61 + 10 * k + j)
+            B.solve(tol=tol)
+            assert max(B.true_residual(k, j) for k, (d, m, n) in enumerate(systems) for j in range(n)) < 1.5 * tol
+            out.append([B.solution(k, j) for k, (d, m, n) in enumerate(systems) for j in range(n)])
+            B.close()
+        assert all(np.array_equal(a, b) for a, b in zip(out[0], out[1]))
