@@ -167,7 +167,7 @@ extern "C" int sfh_upload_gauge(sfh_ctx* c, const double* links)
     if (!c || !links) return SFH_ERR_INVALID;
     cudaSetDevice(c->device);
     size_t n = (size_t)c->g.V * 72 * sizeof(double);
-    int st = cuda_check(c, cudaMemcpyAsync(c->stage, links, n, cudaMemcpyHostToDevice, c->stream), "gauge upload");
+    int st = cuda_check(c, c->copy.in(c->stage, links, n, c->device, c->stream), "gauge upload");
     if (st) return st;
     launch_links_aos_to_eo(c->g, (const double*)c->stage, c->U64, c->stream);
     c->lowp_valid = false;
@@ -180,7 +180,7 @@ extern "C" int sfh_download_gauge(sfh_ctx* c, double* links)
     cudaSetDevice(c->device);
     size_t n = (size_t)c->g.V * 72 * sizeof(double);
     launch_links_eo_to_aos(c->g, c->U64, (double*)c->stage, c->stream);
-    int st = cuda_check(c, cudaMemcpyAsync(links, c->stage, n, cudaMemcpyDeviceToHost, c->stream), "gauge download");
+    int st = cuda_check(c, c->copy.out(links, c->stage, n, c->device, c->stream), "gauge download");
     if (st) return st;
     return cuda_check(c, cudaStreamSynchronize(c->stream), "gauge download");
 }
@@ -188,7 +188,7 @@ extern "C" int sfh_download_gauge(sfh_ctx* c, double* links)
 static int spinor_in(sfh_ctx* c, const double* host, void* eo)
 {
     size_t n = (size_t)c->g.V * 6 * sizeof(double);
-    int st = cuda_check(c, cudaMemcpyAsync(c->stage, host, n, cudaMemcpyHostToDevice, c->stream), "spinor upload");
+    int st = cuda_check(c, c->copy.in(c->stage, host, n, c->device, c->stream), "spinor upload");
     if (st) return st;
     launch_spinor_aos_to_eo(c->g, (const double*)c->stage, eo, c->stream);
     return SFH_OK;
@@ -198,7 +198,7 @@ static int spinor_out(sfh_ctx* c, const void* eo, double* host)
 {
     size_t n = (size_t)c->g.V * 6 * sizeof(double);
     launch_spinor_eo_to_aos(c->g, eo, (double*)c->stage, c->stream);
-    int st = cuda_check(c, cudaMemcpyAsync(host, c->stage, n, cudaMemcpyDeviceToHost, c->stream), "spinor download");
+    int st = cuda_check(c, c->copy.out(host, c->stage, n, c->device, c->stream), "spinor download");
     if (st) return st;
     return cuda_check(c, cudaStreamSynchronize(c->stream), "spinor download");
 }
@@ -289,7 +289,7 @@ extern "C" int sfh_upload_momenta(sfh_ctx* c, const double* P)
     if (!c || !P) return SFH_ERR_INVALID;
     cudaSetDevice(c->device);
     size_t n = (size_t)c->g.V * 72 * sizeof(double);
-    int st = cuda_check(c, cudaMemcpyAsync(c->stage, P, n, cudaMemcpyHostToDevice, c->stream), "momenta upload");
+    int st = cuda_check(c, c->copy.in(c->stage, P, n, c->device, c->stream), "momenta upload");
     if (st) return st;
     launch_links_aos_to_eo(c->g, (const double*)c->stage, c->Pmom, c->stream);
     return cuda_check(c, cudaStreamSynchronize(c->stream), "momenta upload");
@@ -301,7 +301,7 @@ extern "C" int sfh_download_momenta(sfh_ctx* c, double* P)
     cudaSetDevice(c->device);
     size_t n = (size_t)c->g.V * 72 * sizeof(double);
     launch_links_eo_to_aos(c->g, c->Pmom, (double*)c->stage, c->stream);
-    int st = cuda_check(c, cudaMemcpyAsync(P, c->stage, n, cudaMemcpyDeviceToHost, c->stream), "momenta download");
+    int st = cuda_check(c, c->copy.out(P, c->stage, n, c->device, c->stream), "momenta download");
     if (st) return st;
     return cuda_check(c, cudaStreamSynchronize(c->stream), "momenta download");
 }
@@ -373,14 +373,14 @@ extern "C" int sfh_dslash_storage(sfh_ctx* c, int storage, const double* in, dou
     int st = storage_links(c, storage, &U, &gp, &sp);
     if (st) return st;
     const size_t n = (size_t)c->g.V * 6 * sizeof(double);
-    st = cuda_check(c, cudaMemcpyAsync(c->stage, in, n, cudaMemcpyHostToDevice, c->stream), "dslash input");
+    st = cuda_check(c, c->copy.in(c->stage, in, n, c->device, c->stream), "dslash input");
     if (st) return st;
     launch_spinor_aos_to_eo(c->g, (const double*)c->stage, c->spin[0], c->stream);
     launch_spinor_convert(c->g, sp, true, c->spin[0], c->spin[1], c->stream);
     storage_hop(c, storage, U, gp, sp, c->spin[1], c->spin[2], 0, 2);
     launch_spinor_convert(c->g, sp, false, c->spin[2], c->spin[3], c->stream);
     launch_spinor_eo_to_aos(c->g, c->spin[3], (double*)c->stage, c->stream);
-    st = cuda_check(c, cudaMemcpyAsync(out, c->stage, n, cudaMemcpyDeviceToHost, c->stream), "dslash output");
+    st = cuda_check(c, c->copy.out(out, c->stage, n, c->device, c->stream), "dslash output");
     if (st) return st;
     st = cuda_check(c, cudaStreamSynchronize(c->stream), "dslash storage");
     if (st) return st;

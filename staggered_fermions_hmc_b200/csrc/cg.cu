@@ -2477,6 +2477,7 @@ struct sfh_batch {
     int* derr = nullptr;     // device error flags
     sfh::CgWorkspace ws;
     bool ws_ready = false;
+    sfh::HostCopy copy;  // large copies to and from pageable memory
     std::string last_error;
 };
 
@@ -2639,7 +2640,7 @@ extern "C" int sfh_batch_set_gauge(sfh_batch* b, int k, const double* links)
     cudaSetDevice(b->device);
     const sfh::Geom& g = b->geoms[k];
     size_t n = (size_t)g.V * 72 * sizeof(double);
-    int st = batch_cuda(b, cudaMemcpyAsync(b->stage, links, n, cudaMemcpyHostToDevice, b->stream), "gauge upload");
+    int st = batch_cuda(b, b->copy.in(b->stage, links, n, b->device, b->stream), "gauge upload");
     if (st) return st;
     sfh::launch_links_aos_to_eo(g, (const double*)b->stage, b->U64[k], b->stream);
     if (b->prec != SFH_PREC_F64)
@@ -2654,7 +2655,7 @@ extern "C" int sfh_batch_set_rhs(sfh_batch* b, int k, int j, const double* phi)
     cudaSetDevice(b->device);
     const sfh::Geom& g = b->geoms[k];
     size_t n = (size_t)g.V * 6 * sizeof(double);
-    int st = batch_cuda(b, cudaMemcpyAsync(b->stage, phi, n, cudaMemcpyHostToDevice, b->stream), "rhs upload");
+    int st = batch_cuda(b, b->copy.in(b->stage, phi, n, b->device, b->stream), "rhs upload");
     if (st) return st;
     sfh::launch_spinor_aos_to_eo(g, (const double*)b->stage, b->ws.rhs[b->ws.rhs0[k] + j].b, b->stream);
     return batch_cuda(b, cudaStreamSynchronize(b->stream), "rhs convert");
@@ -2681,8 +2682,8 @@ extern "C" int sfh_batch_get_solution(sfh_batch* b, int k, int j, double* X)
     cudaSetDevice(b->device);
     const sfh::Geom& g = b->geoms[k];
     sfh::launch_spinor_eo_to_aos(g, b->ws.rhs[b->ws.rhs0[k] + j].xhi, (double*)b->stage, b->stream);
-    int st = batch_cuda(b, cudaMemcpyAsync(X, b->stage, (size_t)g.V * 6 * sizeof(double),
-                                           cudaMemcpyDeviceToHost, b->stream), "solution download");
+    int st = batch_cuda(b, b->copy.out(X, b->stage, (size_t)g.V * 6 * sizeof(double), b->device, b->stream),
+                        "solution download");
     if (st) return st;
     return batch_cuda(b, cudaStreamSynchronize(b->stream), "solution download");
 }
@@ -2921,13 +2922,13 @@ int sfh::ctx_cg_solve(sfh_ctx* c, const double* phi, double* X, double tol, int 
                       sfh_cg_info* info)
 {
     size_t fs = (size_t)c->g.V * 6 * sizeof(double);
-    cudaError_t e = cudaMemcpyAsync(c->stage, phi, fs, cudaMemcpyHostToDevice, c->stream);
+    cudaError_t e = c->copy.in(c->stage, phi, fs, c->device, c->stream);
     if (e != cudaSuccess) return cuda_check(c, e, "cg upload");
     launch_spinor_aos_to_eo(c->g, (const double*)c->stage, c->spin[3], c->stream);
     int st = ctx_solve_device(c, c->spin[3], c->spin[4], tol, maxit, prec, info);
     if (st != SFH_OK && st != SFH_ERR_NOCONV && st != SFH_ERR_BREAKDOWN) return st;
     launch_spinor_eo_to_aos(c->g, c->spin[4], (double*)c->stage, c->stream);
-    e = cudaMemcpyAsync(X, c->stage, fs, cudaMemcpyDeviceToHost, c->stream);
+    e = c->copy.out(X, c->stage, fs, c->device, c->stream);
     if (e == cudaSuccess) e = cudaStreamSynchronize(c->stream);
     if (e != cudaSuccess) return cuda_check(c, e, "cg download");
     return st;
@@ -2965,8 +2966,8 @@ extern "C" int sfh_batch_get_gauge(sfh_batch* b, int k, double* links)
     cudaSetDevice(b->device);
     const sfh::Geom& g = b->geoms[k];
     sfh::launch_links_eo_to_aos(g, b->U64[k], (double*)b->stage, b->stream);
-    int st = batch_cuda(b, cudaMemcpyAsync(links, b->stage, (size_t)g.V * 72 * sizeof(double),
-                                           cudaMemcpyDeviceToHost, b->stream), "gauge download");
+    int st = batch_cuda(b, b->copy.out(links, b->stage, (size_t)g.V * 72 * sizeof(double), b->device, b->stream),
+                        "gauge download");
     if (st) return st;
     return batch_cuda(b, cudaStreamSynchronize(b->stream), "gauge download");
 }
@@ -2978,8 +2979,8 @@ extern "C" int sfh_batch_get_rhs(sfh_batch* b, int k, int j, double* phi)
     cudaSetDevice(b->device);
     const sfh::Geom& g = b->geoms[k];
     sfh::launch_spinor_eo_to_aos(g, b->ws.rhs[b->ws.rhs0[k] + j].b, (double*)b->stage, b->stream);
-    int st = batch_cuda(b, cudaMemcpyAsync(phi, b->stage, (size_t)g.V * 6 * sizeof(double),
-                                           cudaMemcpyDeviceToHost, b->stream), "rhs download");
+    int st = batch_cuda(b, b->copy.out(phi, b->stage, (size_t)g.V * 6 * sizeof(double), b->device, b->stream),
+                        "rhs download");
     if (st) return st;
     return batch_cuda(b, cudaStreamSynchronize(b->stream), "rhs download");
 }

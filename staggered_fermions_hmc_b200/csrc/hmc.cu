@@ -42,7 +42,7 @@ int take_device_error(sfh_ctx* c, const char* what)
 
 int spinor_in(sfh_ctx* c, const double* host, void* eo)
 {
-    int st = cuda_check(c, cudaMemcpyAsync(c->stage, host, spinor_bytes(c), cudaMemcpyHostToDevice, c->stream),
+    int st = cuda_check(c, c->copy.in(c->stage, host, spinor_bytes(c), c->device, c->stream),
                         "spinor upload");
     if (st) return st;
     launch_spinor_aos_to_eo(c->g, (const double*)c->stage, eo, c->stream);
@@ -52,7 +52,7 @@ int spinor_in(sfh_ctx* c, const double* host, void* eo)
 int spinor_out(sfh_ctx* c, const void* eo, double* host)
 {
     launch_spinor_eo_to_aos(c->g, eo, (double*)c->stage, c->stream);
-    int st = cuda_check(c, cudaMemcpyAsync(host, c->stage, spinor_bytes(c), cudaMemcpyDeviceToHost, c->stream),
+    int st = cuda_check(c, c->copy.out(host, c->stage, spinor_bytes(c), c->device, c->stream),
                         "spinor download");
     if (st) return st;
     return cuda_check(c, cudaStreamSynchronize(c->stream), "spinor download");
@@ -61,7 +61,7 @@ int spinor_out(sfh_ctx* c, const void* eo, double* host)
 int links_out(sfh_ctx* c, const void* eo, double* host)
 {
     launch_links_eo_to_aos(c->g, eo, (double*)c->stage, c->stream);
-    int st = cuda_check(c, cudaMemcpyAsync(host, c->stage, link_bytes(c), cudaMemcpyDeviceToHost, c->stream),
+    int st = cuda_check(c, c->copy.out(host, c->stage, link_bytes(c), c->device, c->stream),
                         "link field download");
     if (st) return st;
     return cuda_check(c, cudaStreamSynchronize(c->stream), "link field download");

@@ -1,0 +1,46 @@
+// hostcopy.h — copies between the device and pageable host memory.
+//
+// The driver moves pageable memory through its own pinned buffer with one host
+// thread, which also takes the page faults of a freshly allocated result.  A
+// large copy is therefore cut into pieces that several threads move through
+// pinned buffers of the context, one each, while the pieces' transfers queue on
+// the context's stream.  With eight threads, ms: a spinor of 32^3 64 (101 MB) to
+// a new array 22 -> 8, its links (1.2 GB) 250 -> 68, and back 108 -> 32; the
+// operator on a spinor of 38 MB, both ways, 10.0 -> 4.5.
+#pragma once
+
+#include <cuda_runtime.h>
+
+#include <cstddef>
+
+namespace sfh {
+
+class HostCopy {
+  public:
+    HostCopy() = default;
+    HostCopy(const HostCopy&) = delete;
+    HostCopy& operator=(const HostCopy&) = delete;
+    ~HostCopy();
+
+    // Host to device, in the stream's order; the host memory may be reused on
+    // return, as with cudaMemcpyAsync from pageable memory.
+    cudaError_t in(void* dev, const void* host, size_t bytes, int device, cudaStream_t stream);
+    // Device to host, in the stream's order; complete on return or, for
+    // pinned memory, once the stream is.
+    cudaError_t out(void* host, const void* dev, size_t bytes, int device, cudaStream_t stream);
+
+  private:
+    static constexpr int kMaxThreads = 8;
+    static constexpr size_t kPiece = (size_t)2 << 20;
+
+    bool ready();
+    void release();
+    template <bool IN>
+    cudaError_t pieces(char* dev, char* host, size_t bytes, int device, cudaStream_t stream);
+
+    int threads_ = 0;  // 0: not set up; < 0: could not be
+    char* pinned_[kMaxThreads] = {};
+    cudaEvent_t ev_[kMaxThreads] = {};  // the last transfer of each buffer
+};
+
+}  // namespace sfh

@@ -8,6 +8,7 @@
 #include <vector>
 
 #include "../../include/sfh.h"
+#include "hostcopy.h"
 #include "sfh_core.cuh"
 
 namespace sfh {
@@ -54,6 +55,8 @@ struct sfh_ctx {
     double hasen_mass = 0.0;       // Hasenbusch heavy mass (0 = one pseudofermion)
     void* hphi = nullptr;          // heavy pseudofermion and its solution (FP64 spinors)
     void* hX = nullptr;
+
+    sfh::HostCopy copy;            // large copies to and from pageable memory
 
     std::string last_error;
 };

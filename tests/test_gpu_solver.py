@@ -688,3 +688,44 @@ def test_fp64_group_widths_agree(sfh):
             out.append([B.solution(k, j) for k, (d, m, n) in enumerate(systems) for j in range(n)])
             B.close()
         assert all(np.array_equal(a, b) for a, b in zip(out[0], out[1]))
+
+
+def test_large_copies_through_pageable_and_pinned_memory_agree(sfh):
+    """Copies from 32 MB on to or from pageable memory go piecewise through
+    several host threads: links, a spinor (36 MB, a partial last piece) and an
+    operator's result equal those through page-locked arrays byte for byte, in
+    two contexts that copy at the same time."""
+    import threading
+
+    import torch
+
+    dims = (32, 32, 32, 24)
+    V = int(np.prod(dims))
+
+    def pinned(a):
+        t = torch.empty(a.size, dtype=torch.float64, pin_memory=True).numpy()
+        t[:] = a
+        return t
+
+    def run(seed, failures):
+        try:
+            rng = np.random.default_rng(seed)
+            U, psi = rng.standard_normal(72 * V), rng.standard_normal(6 * V)
+            lat = sfh.Lattice(dims, 0.2)
+            got = []
+            for array in (lambda a: a, pinned):
+                lat.upload_gauge(array(U))
+                assert np.array_equal(lat.download_gauge(), U)
+                got.append(lat.apply_DDdagger(array(psi)))
+            assert np.array_equal(got[0], got[1])
+            lat.close()
+        except BaseException as e:
+            failures.append(e)
+
+    failures = []
+    threads = [threading.Thread(target=run, args=(s, failures)) for s in (1, 2)]
+    for t in threads:
+        t.start()
+    for t in threads:
+        t.join()
+    assert not failures, failures
