@@ -159,20 +159,11 @@ __device__ __forceinline__ ItemRange item_range(const CgArgs& a, const CgSys& S,
 }
 
 // The kernels of an iteration are chained by programmatic dependencies
-// (ensure_graph): a kernel's blocks may start, as SMs drain, once all blocks
-// of the kernel before it have started.  Up to here a block reads only what
-// does not change during a solve (its work item, system and vector table);
-// the wait ends when the kernel before is complete and its writes are
-// visible.  Its own successor is let go after the wait, so that no more than
-// two kernels of the chain are in flight.  Launched without such a
-// dependency, both instructions do nothing.  Measured, whole solves: six small
-// FP64 systems (36 us per iteration) 22.7 -> 20.9 ms, FP64 16^4 with 4 RHS
-// 17.5 -> 17.0, FP32 24^4 21.6 -> 20.7, FP16 32^3 64 111.8 -> 109.7.
-__device__ __forceinline__ void pdl_begin()
-{
-    asm volatile("griddepcontrol.wait;" ::: "memory");
-    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
-}
+// (ensure_graph, pdl_begin).  Up to pdl_begin a block reads only what does not
+// change during a solve: its work item, system and vector table.  Measured,
+// whole solves: six small FP64 systems (36 us per iteration) 22.7 -> 20.9 ms,
+// FP64 16^4 with 4 RHS 17.5 -> 17.0, FP32 24^4 21.6 -> 20.7, FP16 32^3 64 111.8 ->
+// 109.7.
 
 // Link staging: every thread copies the 8 links of its site (4 forward at
 // the site, 4 backward at its neighbours) into its own columns of shared

@@ -16,12 +16,12 @@
 // four matrices instead of six, and the sides' links meet in the L1), and adds
 // the sides through shared memory.  The products are FMA chains (su3.cuh).
 // Measured on the B200, one thread and whole walks per link -> this: gauge
-// force 363 -> 247 us at 16^4, 2196 -> 1242 us at 24^4 (1399 with the directions
-// of a site far apart in the grid); staples 2470 -> 1417 us;
-// a heatbath sweep 3.57 -> 0.91 ms at 16^4, 18.1 -> 4.1 ms at 24^4.  It runs at
-// 16 TFLOP/s, 0.45 of the FP64 pipe, latency bound on 12 warps per SM (168
-// registers): a third of the stalls are link loads, a fifth each FMA latency
-// and instruction fetch.  A row of the staples per thread (80 registers, 24
+// force 363 -> 228 us at 16^4, 2196 -> 1160 us at 24^4 (1399 with the directions
+// of a site far apart in the grid, 1242 with the links loaded as read-only
+// data); staples 2470 -> 1300 us; a heatbath sweep 3.57 -> 0.60 ms at 16^4, 18.1 ->
+// 3.3 ms at 24^4.  It runs at 17 TFLOP/s, 0.48 of the FP64 pipe, latency bound on
+// 12 warps per SM (168 registers): a third of the stalls are link loads, a
+// fifth each FMA latency and instruction fetch.  A row of the staples per thread (80 registers, 24
 // warps, every link read by three threads) was bound by the L1: 2696 us.
 #include "sfh_internal.h"
 #include "walk.cuh"
@@ -78,7 +78,7 @@ __device__ __forceinline__ M3 side_m(const Side& s)
     M3 o;
 #pragma unroll
     for (int k = 0; k < 9; ++k) {
-        const double2 v = __ldg(b + (size_t)k * s.Vh);
+        const double2 v = b[(size_t)k * s.Vh];
         o.e[k] = {v.x, v.y};
     }
     return o;
@@ -93,7 +93,7 @@ __device__ __forceinline__ M3 side_d(const Side& s)
     for (int i = 0; i < 3; ++i)
 #pragma unroll
         for (int j = 0; j < 3; ++j) {
-            const double2 v = __ldg(b + i * s.rs + j * s.cs);
+            const double2 v = b[i * s.rs + j * s.cs];
             o.e[3 * i + j] = {v.x, __hiloint2double(__double2hiint(v.y) ^ (int)s.conj, __double2loint(v.y))};
         }
     return o;
@@ -169,7 +169,7 @@ __device__ __forceinline__ M3 plane_link(const PlaneSite& s, int a, int dm, int 
     M3 m;
 #pragma unroll
     for (int k = 0; k < 9; ++k) {
-        const double2 v = __ldg(b + (size_t)k * s.Vh);
+        const double2 v = b[(size_t)k * s.Vh];
         m.e[k] = {v.x, v.y};
     }
     return m;
@@ -563,10 +563,42 @@ __device__ __forceinline__ Cx<double> hb_block(const M3& U, const M3& S, int a, 
     return s;
 }
 
-// one subgroup (rows I, J) of the link U with staple sum A = S^dag
-template <int i, int j>
-__device__ __forceinline__ void hb_subgroup(HbRng& r, M3& U, const M3& S, double beta)
+// What the samplers of a block's 32 links draw, as far as it does not depend on
+// the links: for each subgroup, of the first kHbTries attempts at x0 the
+// logarithms' sum and the acceptance variate, and the unit vector that
+// follows if that attempt is the accepted one (an attempt takes two Philox
+// draws, and every subgroup starts anew).
+constexpr int kHbTries = 4;
+struct HbDraws {
+    double l[3][kHbTries][32], r[3][kHbTries][32], v[3][kHbTries][3][32];
+};
+
+// the six warps take two attempts of one subgroup each
+__device__ __forceinline__ void hb_draw(HbDraws& d, HbRng r)
 {
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, sub = warp >> 1;
+    r.tag = 0x48420000u + (unsigned)sub;
+#pragma unroll 1
+    for (int t = 2 * (warp & 1); t < 2 * (warp & 1) + 2; ++t) {
+        r.draw = 2 * t;
+        r.have = 0;
+        const double r1 = 1.0 - r.u(), r2 = 1.0 - r.u(), r3 = 1.0 - r.u();
+        const double c = cospi(2.0 * r2);
+        d.l[sub][t][lane] = log(r1) + c * c * log(r3);
+        d.r[sub][t][lane] = r.u();
+        double v[3];
+        hb_unit<3>(r, v);
+#pragma unroll
+        for (int k = 0; k < 3; ++k) d.v[sub][t][k][lane] = v[k];
+    }
+}
+
+// one subgroup (rows I, J) of the link U with staple sum A = S^dag; r at its
+// first draw
+template <int i, int j>
+__device__ __forceinline__ void hb_subgroup(const HbDraws& d, int sub, HbRng& r, M3& U, const M3& S, double beta)
+{
+    const int lane = threadIdx.x & 31;
     const Cx<double> b0 = hb_block(U, S, i, i), b1 = hb_block(U, S, i, j), b2 = hb_block(U, S, j, i),
                      b3 = hb_block(U, S, j, j);
     const double w0 = 0.5 * (b0.re + b3.re), w1 = 0.5 * (b1.im + b2.im);
@@ -578,9 +610,24 @@ __device__ __forceinline__ void hb_subgroup(HbRng& r, M3& U, const M3& S, double
         hb_unit<4>(r, q);
         quat_su2(q, R);
     } else {
-        const double x0 = hb_x0(r, a, 2.0 * beta / 3.0);
-        double v[3];
-        hb_unit<3>(r, v);
+        const double b = 2.0 * beta / 3.0;
+        double x0 = 0.0, v[3];
+        int t = 0;
+#pragma unroll 1
+        for (; t < kHbTries; ++t) {
+            const double l2 = -1.0 / (2.0 * a * b) * d.l[sub][t][lane];
+            const double x = 1.0 - l2, rr = d.r[sub][t][lane];
+            x0 = 1.0 - 2.0 * l2;
+            if (rr * rr <= x && x >= -1.0 && x <= 1.0) break;
+        }
+        if (t < kHbTries) {
+#pragma unroll
+            for (int k = 0; k < 3; ++k) v[k] = d.v[sub][t][k][lane];
+        } else {
+            r.draw = 2 * kHbTries;
+            x0 = hb_x0(r, a, b);
+            hb_unit<3>(r, v);
+        }
         const double nx = sqrt(1.0 - x0 * x0);
         const double qx[4] = {x0, nx * v[0], nx * v[1], nx * v[2]};
         const double qw[4] = {w0 / a, -w1 / a, -w2 / a, -w3 / a};
@@ -630,47 +677,65 @@ __device__ __forceinline__ Coord hb_site(const Geom& g, int mu, int colour, int 
 // Only the colour's links have threads (one link in eight of a thread per site
 // left every warp an eighth full): six warps share the staples of 32 of them (a
 // launch at 16^4 has 8192 links, 55 per SM, and their staples are a chain of 66
-// products), then one warp updates them: 112 -> 28 us a launch at 16^4, where
-// the three subgroups' sampling loops in one warp are now most of it.
+// products), then one warp updates them: 112 -> 28 us a launch at 16^4.  What the
+// samplers draw needs no link, so all six warps draw it first, while the
+// launch before is still at work: 28 -> 27 us, with the programmatic dependency
+// and plain loads of the links 19; at 4^4 21 -> 10.
 __global__ void __launch_bounds__(kSideThreads, 2) heatbath_kernel(Geom g, void* U, int mu, int colour, double beta,
                                                                    double c11, double c12, unsigned long long seed,
                                                                    int sweep)
 {
     __shared__ SideSum sum;
+    __shared__ HbDraws draws;
     const int k = blockIdx.x * 32 + (threadIdx.x & 31), n = g.V / 8;
     const Coord c = hb_site(g, mu, colour, min(k, n - 1));
     const int p = (c.x[0] + c.x[1] + c.x[2] + c.x[3]) & 1, i = c.lex >> 1;
+    HbRng r;
+    r.key = make_uint2((unsigned)seed, (unsigned)(seed >> 32));
+    r.link = (unsigned)(c.lex * 4 + mu);
+    r.sweep = (unsigned)sweep;
+    hb_draw(draws, r);
+    pdl_begin();  // the draws need no link; plain loads from here, as the links were being written
     M3 S;
     side_staples(U, g, c, p, mu, c11, c12, S, S);
     sum_sides(sum, S);
     if (threadIdx.x >= 32 || k >= n) return;
     S = side_sum(sum);
     M3 u = ld_link(U, p, mu, i, g.Vh);
-    HbRng r;
-    r.key = make_uint2((unsigned)seed, (unsigned)(seed >> 32));
-    r.link = (unsigned)(c.lex * 4 + mu);
-    r.sweep = (unsigned)sweep;
     auto restart = [&](int sub) {
         r.tag = 0x48420000u + (unsigned)sub;
         r.draw = 0;
         r.have = 0;
     };
     restart(0);
-    hb_subgroup<0, 1>(r, u, S, beta);
+    hb_subgroup<0, 1>(draws, 0, r, u, S, beta);
     restart(1);
-    hb_subgroup<0, 2>(r, u, S, beta);
+    hb_subgroup<0, 2>(draws, 1, r, u, S, beta);
     restart(2);
-    hb_subgroup<1, 2>(r, u, S, beta);
+    hb_subgroup<1, 2>(draws, 2, r, u, S, beta);
     st_link(U, p, mu, i, g.Vh, u);
 }
 
 cudaError_t launch_heatbath(const Geom& g, void* U, double beta, double c11, double c12, unsigned long long seed,
                             int sweep0, int nsweeps, cudaStream_t s)
 {
+    // a launch's draws overlap the launch before it (pdl_begin)
+    cudaLaunchAttribute attr;
+    attr.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr.val.programmaticStreamSerializationAllowed = 1;
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3((g.V / 8 + 31) / 32);
+    cfg.blockDim = dim3(kSideThreads);
+    cfg.stream = s;
+    cfg.attrs = &attr;
+    cfg.numAttrs = 1;
     for (int sw = sweep0; sw < sweep0 + nsweeps; ++sw)
         for (int mu = 0; mu < 4; ++mu)
-            for (int col = 0; col < 8; ++col)
-                heatbath_kernel<<<(g.V / 8 + 31) / 32, kSideThreads, 0, s>>>(g, U, mu, col, beta, c11, c12, seed, sw);
+            for (int col = 0; col < 8; ++col) {
+                const cudaError_t e =
+                    cudaLaunchKernelEx(&cfg, heatbath_kernel, g, U, mu, col, beta, c11, c12, seed, sw);
+                if (e != cudaSuccess) return e;
+            }
     return cudaGetLastError();
 }
 

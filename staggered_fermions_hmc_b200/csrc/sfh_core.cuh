@@ -202,6 +202,18 @@ __device__ __forceinline__ void reconstruct_row2(Mat3<R>& U)
     }
 }
 
+// In a kernel launched with a programmatic dependency: its blocks may start, as
+// SMs drain, once all blocks of the kernel before it have started.  Up to here
+// they read only what that kernel does not write; the wait ends when it is
+// complete and its writes are visible.  The kernel's own successor is let go
+// after the wait, so that no more than two kernels of a chain are in flight.
+// Launched without such a dependency, both instructions do nothing.
+__device__ __forceinline__ void pdl_begin()
+{
+    asm volatile("griddepcontrol.wait;" ::: "memory");
+    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+}
+
 // ---------------------------------------------------------------------------
 // storage formats
 // ---------------------------------------------------------------------------

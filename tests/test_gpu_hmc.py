@@ -539,6 +539,28 @@ def test_heatbath_at_unequal_extents(sfh, orc, dims):
     lat.close()
 
 
+@pytest.mark.parametrize("beta", [0.05, 40.0])
+def test_heatbath_at_many_and_few_rejections(sfh, orc, beta):
+    """The samplers' first four attempts are drawn ahead of the staples: weak
+    coupling takes the first, strong coupling rejects most of them and goes on
+    with the fifth.  A sweep at strong coupling amplifies rounding, since every
+    link's staples hold links just updated, so the bound is what the oracle
+    itself makes of links changed by 1e-15: a few times that is the rounding
+    of a staple sum (18 paths of up to five products); another uniform would
+    change its link at order one."""
+    dims = (4, 8, 4, 8)
+    U = orc.random_gauge(dims, 0.6, 195)
+    noise = 1.0 + 1e-15 * np.random.default_rng(196).standard_normal(U.size)
+    lat = sfh.Lattice(dims, 0.1, beta)
+    lat.upload_gauge(U)
+    lat.heatbath_update(n_sweeps=1, seed=31, sweep0=3)
+    ref = orc.heatbath(dims, beta, U, seed=31, nsweeps=1, sweep0=3)
+    moved = rel(orc.heatbath(dims, beta, U * noise, seed=31, nsweeps=1, sweep0=3), ref)
+    assert moved < 1e-6
+    assert rel(lat.download_gauge(), ref) < max(1e-12, 30.0 * moved)
+    lat.close()
+
+
 @pytest.mark.parametrize("dims", [(2, 2, 2, 2), (2, 6, 4, 2), (6, 2, 2, 10), (4, 6, 10, 6)])
 def test_smearing_kernels_at_odd_sizes(sfh, orc, dims):
     """Stout (odd and even level counts end in different buffers), HEX and the
