@@ -220,13 +220,28 @@ __device__ __forceinline__ Mat3<typename GaugeFmt<GP>::R> hop_link(const typenam
     }
 }
 
+// bring a stored link into the L1 ahead of its load
+template <int GP>
+__device__ __forceinline__ void prefetch_link(const void* Ulo, int p, int mu, int i, int Vh)
+{
+    typedef GaugeFmt<GP> F;
+    const typename F::E* b = (const typename F::E*)Ulo + ((size_t)(p * 4 + mu) * F::K) * Vh + i;
+#pragma unroll
+    for (int k = 0; k < F::K; ++k) asm volatile("prefetch.global.L1 [%0];" ::"l"(b + (size_t)k * Vh));
+}
+
 // acc[l] += 1/2 sum_mu eta_mu(x) [bc U_mu(x) in_l(x+mu) - bc U_mu(x-mu)^dag in_l(x-mu)]
 // (the hopping term K, Fermions.cpp:218-247) for the lanes with on[l]; each
 // link is loaded once for all lanes of the block.  The time-wrap signs apply
 // to the input vectors of mu = 3, eta / 2 to the sum of both hops.
 // NST (FP16 only): the neighbour vectors of lane l from its staged range at
 // sn + l * W where it holds them (tstage.cuh), else from global memory.
-template <int GP, int SP, int NB, bool STG, bool COH = false, bool NST = false>
+// PF (FP16): the next direction's links are brought into the L1 meanwhile.
+// Worth its instructions only in the first hop with one or two RHS and no
+// inline reliable updates, where registers are left: 32^3 64, 99 -> 90 us a
+// launch, the solve 56.7 -> 55.5 ms; 24^3 48 with two, 48.3 -> 44.6 us (the
+// vectors too: 92 us; with four RHS 75 -> 97; the second hop spills, 120 -> 123).
+template <int GP, int SP, int NB, bool STG, bool COH = false, bool NST = false, bool PF = false>
 __device__ __forceinline__ void hop_lanes(const void* Ulo, const typename GaugeFmt<GP>::E* sl, const Nbr& n, int q,
                                           int i, int Vh, const void* const (&in)[NB], const bool (&on)[NB],
                                           Vec3<typename GaugeFmt<GP>::R> (&acc)[NB], const uint4* sn = nullptr,
@@ -245,6 +260,12 @@ __device__ __forceinline__ void hop_lanes(const void* Ulo, const typename GaugeF
     if constexpr (GP == GP_F16_12 && SP == SP_F16) {
 #pragma unroll
         for (int mu = 0; mu < 4; ++mu) {
+            if constexpr (PF) {
+                if (mu < 3) {
+                    prefetch_link<GP>(Ulo, q, mu + 1, i, Vh);
+                    prefetch_link<GP>(Ulo, nq, mu + 1, n.dn[mu + 1], Vh);
+                }
+            }
             const float s = ((n.eta >> mu) & 1u) ? -0.5f : 0.5f;
             __half2 U[9];
             hlink_load<STG>(sl, kTile, Ulo, 2 * mu, q, mu, i, Vh, U);
@@ -721,7 +742,8 @@ __device__ __forceinline__ void hop1_item(const CgArgs& a, const int2 it, int cu
             Vec3<R> acc[NB];
 #pragma unroll
             for (int l = 0; l < NB; ++l) vzero(acc[l]);
-            hop_lanes<GP, SP, NB, STG>(S.Ulo, sl, n, q, ti.i, Vh, pin, on, acc);
+            constexpr bool PF = GP == GP_F16_12 && NB <= 2 && !RUI && !STG;
+            hop_lanes<GP, SP, NB, STG, false, false, PF>(S.Ulo, sl, n, q, ti.i, Vh, pin, on, acc);
 #pragma unroll
             for (int l = 0; l < NB; ++l) {
                 if (!on[l]) continue;
