@@ -11,7 +11,7 @@ namespace sfh {
 namespace {
 
 // From here on the first copy repays the buffers (16 MB) and every copy its
-// threads; below, the driver's own takes less than 8 ms.
+// threads; below, CUDA's own copy takes less than 8 ms.
 constexpr size_t kLeastBytes = (size_t)32 << 20;
 
 bool pageable(const void* host)

@@ -1,6 +1,6 @@
 // hostcopy.h — copies between the device and pageable host memory.
 //
-// The driver moves pageable memory through its own pinned buffer with one host
+// The CUDA driver moves pageable memory through its own pinned buffer with one host
 // thread, which also takes the page faults of a freshly allocated result.  A
 // large copy is therefore cut into pieces that several threads move through
 // pinned buffers of the context, one each, while the pieces' transfers queue on

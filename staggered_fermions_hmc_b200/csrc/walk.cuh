@@ -59,14 +59,4 @@ __device__ __forceinline__ M3 link_at(const void* U, const Geom& g, const Walker
     return m;
 }
 
-__device__ __forceinline__ Walker link_coords(const Geom& g, int p, int i)
-{
-    Coord c = eo_coords(g, p, i);
-    Walker w;
-#pragma unroll
-    for (int k = 0; k < 4; ++k) w.x[k] = c.x[k];
-    return w;
-}
-
-
 }  // namespace sfh
