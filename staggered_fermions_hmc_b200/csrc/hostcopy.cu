@@ -24,18 +24,32 @@ bool pageable(const void* host)
     return a.type == cudaMemoryTypeUnregistered;
 }
 
+// a stream under capture keeps the driver's copy and its error
+bool capturing(cudaStream_t stream)
+{
+    cudaStreamCaptureStatus s = cudaStreamCaptureStatusNone;
+    if (cudaStreamIsCapturing(stream, &s) == cudaSuccess) return s != cudaStreamCaptureStatusNone;
+    cudaGetLastError();
+    return true;
+}
+
 }  // namespace
 
 HostCopy::~HostCopy() { release(); }
 
 void HostCopy::release()
 {
+    if (own_) cudaStreamSynchronize(own_);
     for (int k = 0; k < kMaxThreads; ++k) {
         if (ev_[k]) cudaEventDestroy(ev_[k]);
         if (pinned_[k]) cudaFreeHost(pinned_[k]);
         ev_[k] = nullptr;
         pinned_[k] = nullptr;
     }
+    if (order_) cudaEventDestroy(order_);
+    if (own_) cudaStreamDestroy(own_);
+    order_ = nullptr;
+    own_ = nullptr;
 }
 
 bool HostCopy::ready()
@@ -55,11 +69,28 @@ bool HostCopy::ready()
     return true;
 }
 
+// The copy in the order of the caller's stream.  cudaStreamPerThread names
+// another stream in each of the threads: its pieces take a stream of the
+// object's own, after what the caller's holds and before what comes to it next.
+template <bool IN>
+cudaError_t HostCopy::pieces(char* dev, char* host, size_t bytes, int device, cudaStream_t stream)
+{
+    if (stream != cudaStreamPerThread) return move<IN>(dev, host, bytes, device, stream);
+    cudaError_t e;
+    if (!own_ && (e = cudaStreamCreateWithFlags(&own_, cudaStreamNonBlocking)) != cudaSuccess) return e;
+    if (!order_ && (e = cudaEventCreateWithFlags(&order_, cudaEventDisableTiming)) != cudaSuccess) return e;
+    if ((e = cudaEventRecord(order_, stream)) != cudaSuccess) return e;
+    if ((e = cudaStreamWaitEvent(own_, order_, 0)) != cudaSuccess) return e;
+    if ((e = move<IN>(dev, host, bytes, device, own_)) != cudaSuccess) return e;
+    if ((e = cudaEventRecord(order_, own_)) != cudaSuccess) return e;
+    return cudaStreamWaitEvent(stream, order_, 0);
+}
+
 // Each thread takes pieces from a counter and moves them through its own
 // buffer; the calling thread is one of them, so that the copy completes
 // however many others could be started.
 template <bool IN>
-cudaError_t HostCopy::pieces(char* dev, char* host, size_t bytes, int device, cudaStream_t stream)
+cudaError_t HostCopy::move(char* dev, char* host, size_t bytes, int device, cudaStream_t stream)
 {
     std::atomic<size_t> next{0};
     cudaError_t err[kMaxThreads] = {};
@@ -101,14 +132,14 @@ cudaError_t HostCopy::pieces(char* dev, char* host, size_t bytes, int device, cu
 
 cudaError_t HostCopy::in(void* dev, const void* host, size_t bytes, int device, cudaStream_t stream)
 {
-    if (bytes >= kLeastBytes && pageable(host) && ready())
+    if (bytes >= kLeastBytes && pageable(host) && !capturing(stream) && ready())
         return pieces<true>((char*)dev, (char*)const_cast<void*>(host), bytes, device, stream);
     return cudaMemcpyAsync(dev, host, bytes, cudaMemcpyHostToDevice, stream);
 }
 
 cudaError_t HostCopy::out(void* host, const void* dev, size_t bytes, int device, cudaStream_t stream)
 {
-    if (bytes >= kLeastBytes && pageable(host) && ready())
+    if (bytes >= kLeastBytes && pageable(host) && !capturing(stream) && ready())
         return pieces<false>((char*)const_cast<void*>(dev), (char*)host, bytes, device, stream);
     return cudaMemcpyAsync(host, dev, bytes, cudaMemcpyDeviceToHost, stream);
 }

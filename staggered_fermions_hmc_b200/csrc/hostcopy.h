@@ -37,10 +37,14 @@ class HostCopy {
     void release();
     template <bool IN>
     cudaError_t pieces(char* dev, char* host, size_t bytes, int device, cudaStream_t stream);
+    template <bool IN>
+    cudaError_t move(char* dev, char* host, size_t bytes, int device, cudaStream_t stream);
 
     int threads_ = 0;  // 0: not set up; < 0: could not be
     char* pinned_[kMaxThreads] = {};
     cudaEvent_t ev_[kMaxThreads] = {};  // the last transfer of each buffer
+    cudaStream_t own_ = nullptr;        // the pieces' stream for cudaStreamPerThread
+    cudaEvent_t order_ = nullptr;       // orders it against the caller's
 };
 
 }  // namespace sfh

@@ -729,3 +729,26 @@ def test_large_copies_through_pageable_and_pinned_memory_agree(sfh):
     for t in threads:
         t.join()
     assert not failures, failures
+
+
+def test_large_copies_on_a_per_thread_stream(sfh):
+    """cudaStreamPerThread names another stream in every host thread, and large
+    copies to and from pageable memory run on several: uploads land before the
+    kernels queued after them, downloads start after the kernels before them,
+    so that new links come back byte for byte, round after round, in a context
+    and in a batch (36 MB each way, the copies' threshold is 32 MB)."""
+    import ctypes
+
+    per_thread, dims = ctypes.c_void_p(2), (16, 16, 16, 16)
+    rng = np.random.default_rng(5)
+    lat, B = sfh.Lattice(dims, 0.2), sfh.Batch([(dims, 0.2, 1)], precision="f64")
+    assert lat.lib.sfh_set_stream(lat.h, per_thread) == 0
+    assert B.lib.sfh_batch_set_stream(B.h, per_thread) == 0
+    for _ in range(10):
+        U = rng.standard_normal(72 * 16 ** 4)
+        lat.upload_gauge(U)
+        assert np.array_equal(lat.download_gauge(), U)
+        B.set_gauge(0, U)
+        assert np.array_equal(B.gauge(0), U)
+    lat.close()
+    B.close()
