@@ -1074,7 +1074,9 @@ cudaError_t flow_launch(int prec, const CgArgs& a, const FlowArgs& f, const Flow
                      : prec == SFH_PREC_F16    ? f16[sl]
                      : prec == SFH_PREC_F32_18 ? cg_flow<GP_F32_18, SP_F32, 1, false>
                                                : cg_flow<GP_BF16_12, SP_BF16, 1, false>;
-    cudaError_t e = cudaFuncSetAttribute((const void*)k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)plan.dyn);
+    // the same limit from every handle: it belongs to the kernel, and another
+    // thread may be about to launch it with more than this plan takes
+    cudaError_t e = cudaFuncSetAttribute((const void*)k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kFlowMaxSmem);
     if (e != cudaSuccess) return e;
     CgArgs ca = a;
     FlowArgs fa = f;

@@ -752,3 +752,46 @@ def test_large_copies_on_a_per_thread_stream(sfh):
         assert np.array_equal(B.gauge(0), U)
     lat.close()
     B.close()
+
+
+@pytest.mark.parametrize("precision,systems,schedule", [
+    ("f64", [((12, 12, 12, 12), 0.1, 1), ((16, 16, 16, 16), 0.1, 1)], (0, 0, 0)),  # the dataflow kernel, 1 and 3 rounds of sites
+    ("f16", [((8, 8, 8, 4), 0.1, 2), ((8, 8, 8, 64), 0.1, 2)], (2, 2, 6)),         # staged ranges of 260 and 320 vectors
+])
+def test_handles_in_threads_share_kernels_of_other_shared_memory(sfh, precision, systems, schedule):
+    """Handles in threads of their own launch the same kernel with unequal
+    amounts of shared memory, many times at once: none changes what another
+    may use (a kernel's limit belongs to the kernel, not to the handle), every
+    solve ends as alone, and the results are those of a solve alone.  The
+    iteration limit changes from solve to solve, so that each builds its graph."""
+    import threading
+
+    def make(k):
+        B = sfh.Batch([systems[k]], precision=precision)
+        B.set_schedule(*schedule)
+        B.random_gauge(0, 0.5, 21 + k)
+        for j in range(systems[k][2]):
+            B.random_rhs(0, j, 31 + k + 10 * j)
+        return B
+
+    def solve(B, max_iter=1):
+        return B.solve(tol=1e-10, max_iter=max_iter, check=False)
+
+    batches = [make(k % 2) for k in range(8)]
+    alone = [(solve(B), B.solution(0, 0)) for B in batches[:2]]
+    seen = [[] for B in batches]
+
+    def run(k):
+        for i in range(500):
+            seen[k].append(solve(batches[k], 2 - i % 2))
+
+    threads = [threading.Thread(target=run, args=(k,)) for k in range(8)]
+    for t in threads:
+        t.start()
+    for t in threads:
+        t.join()
+    for k, B in enumerate(batches):
+        assert alone[k % 2][0] == sfh.SFH_ERR_NOCONV
+        assert set(seen[k]) == {sfh.SFH_ERR_NOCONV}, B.lib.sfh_batch_last_error(B.h)
+        assert np.array_equal(B.solution(0, 0), alone[k % 2][1])
+        B.close()
