@@ -615,7 +615,7 @@ class Batch:
 
     def set_barrier_polls(self, polls):
         """Bound on each grid-barrier wait of the persistent schedule (0: the
-        default, about 4 s)."""
+        default, about 4 s) and on each wait of the dataflow launch."""
         self._check(self.lib.sfh_batch_set_barrier_polls(self.h, int(polls)), "set_barrier_polls")
 
     def set_reliable_delta(self, delta):

@@ -44,6 +44,7 @@
 // FP64 true residual.
 #include <algorithm>
 #include <chrono>
+#include <climits>
 #include <cmath>
 #include <cstring>
 #include <string>
@@ -1735,7 +1736,7 @@ struct CgWorkspace {
     int* d_rulist = nullptr;   // reliable-update lane lists [2][1 + nlanes]
     int* d_qctr = nullptr;     // work-item counters of schedule 7 [2][2]
     bool timed_out = false;    // the last persistent solve gave up at a barrier
-    long long barrier_polls = 0;  // bound on each barrier wait (0: the default)
+    long long barrier_polls = 0;  // bound on each barrier or dataflow wait (0: the default)
     int num_sms = 0;
     int auto_nb = 0;           // RHS-block width without an explicit schedule (0: from the RHS count)
     std::vector<void*> allocs;
@@ -2163,7 +2164,7 @@ static cudaError_t flow_solve(CgWorkspace& w, const CgArgs& a, cudaStream_t stre
     f.flags = (unsigned*)(F.d_words + F.flags_at);
     f.pub = F.d_pub_ptr;
     f.err = &w.d_bar->err;
-    f.polls = kFlowPolls;  // about 0.6 us each
+    f.polls = w.barrier_polls > 0 ? (int)std::min<long long>(w.barrier_polls, INT_MAX) : kFlowPolls;
     if ((e = flow_launch(w.prec, a, f, F.plan, stream)) != cudaSuccess) return e;
     w.launches += 1;
     int err = 0;
@@ -2265,11 +2266,13 @@ static AutoSchedule auto_schedule(const CgWorkspace& w)
 // two hop kernels (0 = from the largest RHS count); tpi: tiles per block of
 // the iteration kernels (0 = default_tpi); stage: hop kernels stage their
 // links in shared memory (reduced precisions only); all of them 0:
-// auto_schedule; prefer_flow: the dataflow
-// kernel where the systems suit it, whatever the schedule.  Returns a cudaError.
+// auto_schedule; use: which solves the dataflow kernel takes where the systems
+// suit it (those with all of it 0, all, none).  Returns a cudaError.
+enum FlowUse { FLOW_OPEN, FLOW_PREFER, FLOW_NEVER };
+
 static cudaError_t workspace_solve(CgWorkspace& w, double tol, int maxit, double delta, int nb1, int nb2,
                                    int tpi, int stage, cudaStream_t stream, PhaseTimes* timing = nullptr,
-                                   bool prefer_flow = false)
+                                   FlowUse use = FLOW_OPEN)
 {
     int max_nrhs = 1;
     for (const CgSys& S : w.sys) max_nrhs = std::max(max_nrhs, S.nrhs);
@@ -2278,14 +2281,14 @@ static cudaError_t workspace_solve(CgWorkspace& w, double tol, int maxit, double
     // take the dataflow kernel (flow_plan says where the line lies)
     bool flow = false;
     const bool open = nb1 <= 0 && nb2 <= 0 && tpi <= 0 && stage == 0;
-    if (!timing && (prefer_flow || open)) {
+    if (!timing && use != FLOW_NEVER && (use == FLOW_PREFER || open)) {
         if (w.flow.state == 0) {
             const cudaError_t fe = flow_prepare(w);
             if (fe != cudaSuccess) return fe;
         }
         flow = w.flow.state > 0;
     }
-    if (open && !prefer_flow) {
+    if (open && use != FLOW_PREFER) {
         const AutoSchedule s = auto_schedule(w);
         nb1 = s.nb1;
         nb2 = s.nb2;
@@ -2360,9 +2363,18 @@ static cudaError_t workspace_solve(CgWorkspace& w, double tol, int maxit, double
     if ((e = cudaGetLastError()) != cudaSuccess) return e;
     if (flow) {
         e = flow_solve(w, a, stream);
-        if (e != cudaErrorCooperativeLaunchTooLarge) return e;
-        cudaGetLastError();  // fewer SMs than the device reports: the per-phase kernels
-        w.flow.state = -1;
+        if (e == cudaErrorCooperativeLaunchTooLarge) {  // fewer SMs than the device reports
+            cudaGetLastError();
+            w.flow.state = -1;
+        } else if (e != cudaSuccess || !w.timed_out) {
+            return e;
+        }
+        // not launched, or a wait of it gave up: the per-phase kernels, from
+        // the right-hand sides again
+        const long before = w.launches;
+        e = workspace_solve(w, tol, maxit, delta, nb1, nb2, tpi, stage, stream, nullptr, FLOW_NEVER);
+        w.launches += before;
+        return e;
     }
     if (k.pers) return persistent_solve(w, k, a, stream, timing);
     if (!timing && (e = ensure_graph(w, k, a, tol, maxit, delta)) != cudaSuccess) return e;
@@ -2677,7 +2689,7 @@ extern "C" int sfh_batch_solve(sfh_batch* b, double tol, int maxit)
     if (!b || !(tol > 0.0) || maxit <= 0) return SFH_ERR_INVALID;
     cudaSetDevice(b->device);
     int st = batch_cuda(b, sfh::workspace_solve(b->ws, tol, maxit, b->delta, b->nb, b->nb2, b->tpi, b->stage_links, b->stream,
-                                                nullptr, b->tuned_flow), "batched CG");
+                                                nullptr, b->tuned_flow ? sfh::FLOW_PREFER : sfh::FLOW_OPEN), "batched CG");
     if (st) return st;
     if (b->ws.timed_out)
         return batch_err(b, SFH_ERR_TIMEOUT, "batched CG: a bounded device wait (grid barrier or neighbour staging) gave up");
@@ -3069,7 +3081,8 @@ extern "C" int sfh_batch_autotune(sfh_batch* b, int probe_iters, int* best_width
     double flow = 1e300;
     for (int rep = 0; rep < 2 && b->ws.flow.state >= 0; ++rep) {
         auto t0 = std::chrono::steady_clock::now();
-        cudaError_t e = sfh::workspace_solve(b->ws, 1e-30, probe_iters, 0.1, bw, bw2, bt, bs, b->stream, nullptr, true);
+        cudaError_t e = sfh::workspace_solve(b->ws, 1e-30, probe_iters, 0.1, bw, bw2, bt, bs, b->stream, nullptr,
+                                             sfh::FLOW_PREFER);
         if (e != cudaSuccess) return batch_cuda(b, e, "autotune");
         if (b->ws.flow.state > 0)
             flow = std::chrono::duration<double>(std::chrono::steady_clock::now() - t0).count();

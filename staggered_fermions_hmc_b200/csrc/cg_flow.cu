@@ -28,8 +28,8 @@
 // of FP32 site products, so that their solutions equal the per-phase kernels'
 // unless a sum's last bit turns the FP32 rounding of alpha or beta.  An FP64
 // reliable update runs on the global arrays between two fenced team barriers.
-// Every wait is bounded; one that gives up sets the error word, and the others
-// follow.
+// Every wait is bounded; one that gives up sets the error word, the others
+// follow, and the solve runs again in the per-phase kernels.
 //
 // Measured, us per iteration, per-phase kernels -> this one: FP64 4^4 15 -> 6,
 // 8^3 16 20 -> 8.5, 12^4 21 -> 12.7, 16^4 26 -> 21.5, 16^3 32 58 -> 53; FP32

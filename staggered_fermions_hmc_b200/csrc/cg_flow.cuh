@@ -45,6 +45,6 @@ bool flow_plan(const std::vector<CgSys>& sys, int prec, int num_sms, FlowPlan* p
 // the whole solve (after cg_init) in one cooperative launch
 cudaError_t flow_launch(int prec, const CgArgs& a, const FlowArgs& f, const FlowPlan& plan, cudaStream_t stream);
 
-constexpr int kFlowPolls = 1 << 22;  // bound on each wait
+constexpr int kFlowPolls = 1 << 22;  // bound on each wait, about 0.6 us a poll
 
 }  // namespace sfh

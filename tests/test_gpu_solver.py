@@ -795,3 +795,46 @@ def test_handles_in_threads_share_kernels_of_other_shared_memory(sfh, precision,
         assert set(seen[k]) == {sfh.SFH_ERR_NOCONV}, B.lib.sfh_batch_last_error(B.h)
         assert np.array_equal(B.solution(0, 0), alone[k % 2][1])
         B.close()
+
+
+@pytest.mark.parametrize("precision", ["f64", "f32", "f16"])
+def test_dataflow_wait_runs_out_and_the_solve_starts_over(sfh, orc, precision):
+    """With the bound on the dataflow kernel's waits cut to one poll a launch
+    of several blocks gives up; the solve then runs in the per-phase kernels
+    from the same right-hand sides: SFH_OK, the solutions of an explicit
+    schedule bit for bit, the oracle's true residual.  With the default bound
+    the next solve of the batch is the dataflow launch's again."""
+    systems, tol = [((8, 8, 8, 8), 0.1, 2), ((6, 6, 6, 8), 0.2, 1)], 1e-10
+    fields = [(orc.random_gauge(d, 0.5, 81 + k), [orc.random_spinor(d, 91 + 10 * k + j) for j in range(n)])
+              for k, (d, m, n) in enumerate(systems)]
+
+    def batch(schedule):
+        B = sfh.Batch(systems, precision=precision)
+        B.set_schedule(*schedule)
+        for k, (U, bs) in enumerate(fields):
+            B.set_gauge(k, U)
+            for j, b in enumerate(bs):
+                B.set_rhs(k, j, b)
+        return B
+
+    def solve(B):
+        B.solve(tol=tol)
+        return [B.solution(k, j) for k, (d, m, n) in enumerate(systems) for j in range(n)]
+
+    B, explicit = batch((0, 0, 0)), batch((1, 1, 0))
+    first = solve(B)
+    assert B.kernel_launches() == 2
+    B.set_barrier_polls(1)
+    again = solve(B)
+    assert B.kernel_launches() > 3  # cg_init and the launch that gave up, then cg_init and the iterations' kernels
+    assert all(np.array_equal(a, b) for a, b in zip(again, solve(explicit)))
+    at = 0
+    for (dims, mass, nrhs), (U, bs) in zip(systems, fields):
+        for b in bs:
+            assert true_resid(orc, dims, mass, U, b, again[at]) < 1.5 * tol
+            at += 1
+    B.set_barrier_polls(0)
+    assert all(np.array_equal(a, b) for a, b in zip(solve(B), first))
+    assert B.kernel_launches() == 2
+    B.close()
+    explicit.close()
