@@ -336,10 +336,15 @@ int sfh_batch_get_hop_widths(sfh_batch* batch, int* hop1_width, int* hop2_width)
  * (1, 2, 4, 8; FP64: 1, 2), tiles-per-block count (1, 2, 4) and link staging
  * (0 to 7 as below; FP64: 0; 6 for FP16 only), and for the lane-list stages
  * (4 to 7) also hop widths 4 and 2, on the batch's current inputs and keep
- * the fastest; where the dataflow launch of small batches is faster still, it
- * runs the solves until a schedule is set.
- * The schedule never changes the results.  No counterpart in the reference
- * (its solver has no schedule). */
+ * the fastest.  The schedule does not change the mixed precisions' results;
+ * FP64's sums are added per block, so that the tiles per block turn their last
+ * bits.  Small batches whose solves take the dataflow launch without a
+ * schedule (sfh_batch_set_schedule) go on taking it where it is the faster one
+ * by the sizes (one RHS per system: up to 768 sites per SM and parity, 384 in
+ * FP64; with more RHS fewer), never by the timings, until a schedule is
+ * set; sfh_batch_get_schedule then gives the fastest schedule all the same,
+ * and setting it selects that schedule's kernels.  No counterpart in the
+ * reference (its solver has no schedule). */
 int sfh_batch_autotune(sfh_batch* batch, int probe_iters, int* best_width);
 /* The schedule directly: RHS-block width (0 = automatic), 256-site tiles per
  * block of the iteration kernels (0 = 2, or 1 where two would give the first
@@ -408,8 +413,10 @@ int sfh_batch_kernel_launches(sfh_batch* batch, long* n);
  * t = K p; v = m^2 p - K t with the CG sums; the x, r, p update; with the
  * system-blocked schedule the two FP64 reliable-update kernels (zero
  * otherwise: the hop kernels do those hops); and with the persistent schedule
- * the one cooperative launch (the others zero).  Same kernels, same results;
- * a measurement aid with no counterpart in the reference. */
+ * the one cooperative launch (the others zero).  The kernels and results of
+ * sfh_batch_solve, but for small batches whose solves take the dataflow
+ * launch: there the kernels of the schedule are timed, whose sums are added in
+ * another order.  A measurement aid with no counterpart in the reference. */
 #define SFH_TIMED_KERNELS 6
 int sfh_batch_solve_timed(sfh_batch* batch, double tol, int maxit, double* ms, long* n);
 /* FP64 |b - D D^dag x| / |b| for one solution (diagnostic) */

@@ -580,8 +580,9 @@ class Batch:
         return a.value, b.value
 
     def autotune(self, probe_iters=48):
-        """Pick the fastest RHS-block width and tiles per block for this batch
-        (schedule only); returns the width."""
+        """Pick the fastest RHS-block width, tiles per block and link staging for
+        this batch; returns the width.  Small batches keep the dataflow launch,
+        by their sizes and not by the timings."""
         w = ctypes.c_int(0)
         self._check(self.lib.sfh_batch_autotune(self.h, probe_iters, ctypes.byref(w)), "autotune")
         return w.value
@@ -590,7 +591,8 @@ class Batch:
         """Solve with per-kernel CUDA-event timing; returns {kernel: (ms, launches)}
         for the kernels the schedule launched (the reliable-update kernels
         cg_ru1 / cg_ru2 with the system-blocked schedule only; cg_persistent
-        alone with the persistent schedule)."""
+        alone with the persistent schedule).  Small batches, which solve() runs
+        in the dataflow launch, are timed in the schedule's kernels."""
         ms = np.zeros(TIMED_KERNELS)
         n = (ctypes.c_long * TIMED_KERNELS)()
         self._check(self.lib.sfh_batch_solve_timed(self.h, tol, max_iter, _dptr(ms), n), "solve_timed")

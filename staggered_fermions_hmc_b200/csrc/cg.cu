@@ -26,7 +26,8 @@
 // Work is split into tiles of 256 sites of one system and one output parity.
 // A work item is a range of tiles and a group of the system's RHS, so a link
 // loaded once serves every RHS of the group (RHS blocking).  Schedules (the
-// autotuner times them; results never depend on the choice): links read
+// autotuner times them; the mixed precisions' results do not depend on the
+// choice, FP64's only on the tiles per item, whose sums are added first): links read
 // directly or staged per work item; the FP64 reliable-update hops inside the
 // hop kernels or in two kernels walking a device list of the lanes due for
 // one; system-blocked kernels (one tile per block, every RHS of the system,
@@ -2488,7 +2489,7 @@ struct sfh_batch {
     cudaStream_t stream = nullptr;
     bool own_stream = false;
     int prec = 0, flags = 0, nb = 0, nb2 = 0, tpi = 0, stage_links = 0;
-    bool tuned_flow = false;  // the autotuner found the dataflow kernel faster than its schedule
+    bool tuned_flow = false;  // autotuned, and small enough for the dataflow kernel
     double delta = 0.1;  // reliable-update threshold of the mixed precisions (set at creation)
     std::vector<sfh_system_desc> desc;
     std::vector<sfh::Geom> geoms;
@@ -3037,8 +3038,10 @@ extern "C" int sfh_batch_kernel_launches(sfh_batch* b, long* n)
 
 // Autotuner: times a capped solve (probe_iters iterations, no lane converges)
 // for every RHS-block width, tiles-per-block count and link staging mode
-// (read directly, staged per work item, system-blocked), and the dataflow
-// kernel, and keeps the fastest.
+// (read directly, staged per work item, system-blocked) and keeps the
+// fastest.  Whether the solves take the dataflow kernel, which adds its sums in
+// another order, is not left to the timing: a program's results would change
+// from run to run.
 extern "C" int sfh_batch_autotune(sfh_batch* b, int probe_iters, int* best_width)
 {
     if (!b || probe_iters < 1) return SFH_ERR_INVALID;
@@ -3077,17 +3080,11 @@ extern "C" int sfh_batch_autotune(sfh_batch* b, int probe_iters, int* best_width
                     bs = stage;
                 }
             }
-    // the dataflow kernel against the fastest schedule, which stays the batch's
-    double flow = 1e300;
-    for (int rep = 0; rep < 2 && b->ws.flow.state >= 0; ++rep) {
-        auto t0 = std::chrono::steady_clock::now();
-        cudaError_t e = sfh::workspace_solve(b->ws, 1e-30, probe_iters, 0.1, bw, bw2, bt, bs, b->stream, nullptr,
-                                             sfh::FLOW_PREFER);
+    if (b->ws.flow.state == 0) {
+        const cudaError_t e = sfh::flow_prepare(b->ws);
         if (e != cudaSuccess) return batch_cuda(b, e, "autotune");
-        if (b->ws.flow.state > 0)
-            flow = std::chrono::duration<double>(std::chrono::steady_clock::now() - t0).count();
     }
-    b->tuned_flow = flow < best;
+    b->tuned_flow = b->ws.flow.state > 0 && sfh::flow_beats_tuned(b->ws.sys, b->ws.flow.plan);
     b->nb = bw;
     b->nb2 = bw2;
     b->tpi = bt;

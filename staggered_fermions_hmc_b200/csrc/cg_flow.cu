@@ -1050,11 +1050,24 @@ bool flow_plan(const std::vector<CgSys>& sys, int prec, int num_sms, FlowPlan* p
     };
     if (prec == SFH_PREC_F64 || prec == SFH_PREC_F32 || prec == SFH_PREC_F16)
         while (plan->split < 4 && 64 * warps(2 * plan->split) <= most) plan->split *= 2;
-    const int all = warps(plan->split), rounds = (64 * all + most - 1) / most;
-    plan->threads = 64 * ((all + rounds - 1) / rounds);
-    plan->one = rounds == 1;
+    const int all = warps(plan->split);
+    plan->rounds = (64 * all + most - 1) / most;
+    plan->threads = 64 * ((all + plan->rounds - 1) / plan->rounds);
+    plan->one = plan->rounds == 1;
     if (plan->dyn > kFlowMaxSmem) return false;
     return true;
+}
+
+// By the rounds of a hop, which serve the RHS of a block one after the other
+// where the per-phase kernels share a link's load.  Best schedule / dataflow,
+// five precisions: one RHS, three rounds 1.01 to 1.24, four 1.00; two to four
+// RHS, two rounds 1.03 to 1.23, three 0.91 to 1.17; five to eight RHS, one round
+// 1.08 to 1.38, two 0.86 to 1.07.
+bool flow_beats_tuned(const std::vector<CgSys>& sys, const FlowPlan& plan)
+{
+    int most = 1;
+    for (const CgSys& S : sys) most = std::max(most, S.nrhs);
+    return plan.rounds <= (most == 1 ? 3 : (most <= 4 ? 2 : 1));
 }
 
 cudaError_t flow_launch(int prec, const CgArgs& a, const FlowArgs& f, const FlowPlan& plan, cudaStream_t stream)

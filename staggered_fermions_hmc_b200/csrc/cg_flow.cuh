@@ -36,12 +36,15 @@ struct FlowPlan {
     size_t words = 0, pub_bytes = 0;
     int threads = 0;
     int split = 1;                 // threads per site in a hop
-    bool one = false;              // a hop takes one round of the block's threads
+    int rounds = 1;                // of the block's threads, for a hop
+    bool one = false;              // rounds == 1
     size_t dyn = 0;                // dynamic shared memory of a block
 };
 // false where the per-phase kernels are the better ones (or the systems do
 // not fit); host arithmetic only
 bool flow_plan(const std::vector<CgSys>& sys, int prec, int num_sms, FlowPlan* plan);
+// whether such a plan beats the best of the per-phase kernels' schedules too
+bool flow_beats_tuned(const std::vector<CgSys>& sys, const FlowPlan& plan);
 // the whole solve (after cg_init) in one cooperative launch
 cudaError_t flow_launch(int prec, const CgArgs& a, const FlowArgs& f, const FlowPlan& plan, cudaStream_t stream);
 

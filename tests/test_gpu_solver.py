@@ -838,3 +838,42 @@ def test_dataflow_wait_runs_out_and_the_solve_starts_over(sfh, orc, precision):
     assert B.kernel_launches() == 2
     B.close()
     explicit.close()
+
+
+@pytest.mark.parametrize("precision,systems,flow", [
+    ("f64", [((8, 8, 8, 8), 0.2, 2)], True),
+    ("f16", [((8, 8, 8, 8), 0.2, 8)], True),     # one round of a hop
+    ("f32", [((16, 16, 20, 30), 0.2, 1)], True),  # three rounds, one RHS
+    ("f32", [((12, 12, 12, 12), 0.2, 5)], False),  # two rounds, five RHS
+    ("f32_18", [((12, 12, 12, 12), 0.2, 6)], False),  # three rounds, six RHS
+    ("f64", [((16, 16, 16, 32), 0.2, 1)], False),  # four rounds
+    ("f16", [((24, 24, 24, 24), 0.2, 1)], False),  # no dataflow plan
+])
+def test_autotuned_batches_take_the_dataflow_launch_by_size(sfh, precision, systems, flow):
+    """Which kernels an autotuned batch runs, and with them the order of its
+    sums, is decided by its sizes: small batches keep the dataflow launch and
+    the default's solutions bit for bit, larger ones take the tuned schedule,
+    whose solutions are those of the same schedule set by hand."""
+    def batch():
+        B = sfh.Batch(systems, precision=precision)
+        B.random_gauge(0, 0.5, 7)
+        for j in range(systems[0][2]):
+            B.random_rhs(0, j, 17 + j)
+        return B
+
+    def solve(B):
+        B.solve(tol=1e-10)
+        return [B.solution(0, j) for j in range(systems[0][2])]
+
+    B, other = batch(), batch()
+    B.autotune(probe_iters=8)
+    tuned = solve(B)
+    if flow:
+        assert B.kernel_launches() == 2
+    else:
+        assert B.kernel_launches() > 2 or B.schedule()[2] == 3  # 3: one persistent launch
+        other.set_schedule(*B.schedule())
+        other.set_hop_widths(*B.hop_widths())
+    assert all(np.array_equal(a, b) for a, b in zip(tuned, solve(other)))
+    B.close()
+    other.close()
