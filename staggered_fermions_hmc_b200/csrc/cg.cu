@@ -2200,12 +2200,17 @@ static cudaError_t flow_solve(CgWorkspace& w, const CgArgs& a, cudaStream_t stre
 // 19.0; 32^4 32.9, 30.1, 32.5; 32^3 64 61.6, 58.2, 56.9; BF16 24^3 32 14.5, 14.3,
 // 15.9; 28^4 21.3, 20.1, 22.3; 32^4 38.2, 32.6, 32.6; 32^3 64 74.9, 61.5, 60.4.
 //
-// One RHS, FP32: the tiles per item and the staging of least cost, counted in
-// tile times of an SM: B = ceil(items / SMs) blocks of `tiles` tiles each, four
-// for every wave of resident blocks (launch, descriptors, partial last wave) and
-// three for the two more kernels of the lane lists.  Against two tiles and
-// inline updates, ms: 24^3 32 16.2 -> 13.6, 32^4 39.7 -> 30.9, 32^3 64 76.3 ->
-// 69.3.  FP32 18-real gained nothing anywhere.
+// One RHS, FP32: the tiles per item and the staging of least cost, in tile
+// times: every wave of resident blocks, a partial one too, takes its tiles and
+// one more (launch, descriptors, first loads), the two more kernels of the lane
+// lists half of one.  So an item has the fewest tiles that still make one wave of
+// the lattice, and of two ways the one with fewer waves wins.  Against two tiles
+// and inline updates, ms: 20^3 32 (1000 tiles) 10.4 -> 9.1 (two tiles and lane
+// lists, one wave; four tiles inline, which leave a third of the blocks idle,
+// 11.8), 24^4 13.1 -> 12.3, 22x24x26x36 21.7 -> 16.7, 28^4 24.2 -> 23.8, 32^4
+// 40.3 -> 32.7, 28x32x32x48 52.9 -> 52.6 (best: 50.0), 32^3 64 79.2 -> 72.4; the
+// fastest of eight at 24 of 26 sizes from 20^3 32 on.  FP32 18-real gained nothing
+// anywhere.
 struct AutoSchedule {
     int nb1 = 0, nb2 = 0, tpi = 0, stage = 0;
 };
@@ -2251,9 +2256,8 @@ static AutoSchedule auto_schedule(const CgWorkspace& w)
         for (int tpi : {1, 2, 4, 8}) {
             const int occ = stage == 0 ? HopOcc<GP_F32_12, SP_F32, 1, true, true>::v
                                        : HopOcc<GP_F32_12, SP_F32, 1, true, false>::v;
-            const int items = 2 * ((tiles / 2 + tpi - 1) / tpi), B = (items + sms - 1) / sms;
-            // a block alone on its SM does not keep it busy
-            const int cost = std::max(B, 2) * tpi + 4 * ((B + occ - 1) / occ) + (stage ? 3 : 0);
+            const int items = 2 * ((tiles / 2 + tpi - 1) / tpi), waves = (items + occ * sms - 1) / (occ * sms);
+            const int cost = 2 * waves * (tpi + 1) + (stage ? 1 : 0);
             if (cost < best || (cost == best && stage == s.stage)) {
                 best = cost;
                 s.tpi = tpi;

@@ -877,3 +877,22 @@ def test_autotuned_batches_take_the_dataflow_launch_by_size(sfh, precision, syst
     assert all(np.array_equal(a, b) for a, b in zip(tuned, solve(other)))
     B.close()
     other.close()
+
+
+@pytest.mark.parametrize("dims,tiles,stage", [((20, 20, 20, 32), 2, 4), ((24, 24, 24, 24), 4, 0), ((22, 24, 26, 36), 4, 4)])
+def test_f32_solves_without_a_schedule_fill_whole_waves(sfh, dims, tiles, stage):
+    """FP32 solves of one right-hand side above the dataflow launch's sizes
+    take the tiles per item and the staging that need the fewest waves of
+    resident blocks: the launches of that schedule, and its solution bit for
+    bit (every schedule's; 4: two more kernels per iteration)."""
+    out = []
+    for schedule in ((0, 0, 0), (1, tiles, stage)):
+        B = sfh.Batch([(dims, 0.3, 1)], precision="f32")
+        B.set_schedule(*schedule)
+        B.random_gauge(0, 0.5, 3)
+        B.random_rhs(0, 0, 4)
+        B.solve(tol=1e-10)
+        out.append((B.kernel_launches(), B.solution(0, 0)))
+        B.close()
+    assert out[0][0] == out[1][0]
+    assert np.array_equal(out[0][1], out[1][1])
