@@ -1055,7 +1055,13 @@ bool flow_plan(const std::vector<CgSys>& sys, int prec, int num_sms, FlowPlan* p
     plan->threads = 64 * ((all + plan->rounds - 1) / plan->rounds);
     plan->one = plan->rounds == 1;
     if (plan->dyn > kFlowMaxSmem) return false;
-    return true;
+    // FP64 serves the RHS of a block one after the other, round by round, where
+    // the per-phase kernels take a link for two: from five rounds on, with more
+    // than four RHS from four on, these are the faster ones (12^4 with 6 RHS
+    // 6.9 ms against 5.8, with 5 5.8 against 5.4; 16^4 with 2 6.0 against 6.1)
+    int rhs = 1;
+    for (const CgSys& S : sys) rhs = std::max(rhs, S.nrhs);
+    return prec != SFH_PREC_F64 || plan->rounds <= (rhs > 4 ? 3 : 4);
 }
 
 // By the rounds of a hop, which serve the RHS of a block one after the other

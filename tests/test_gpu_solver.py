@@ -896,3 +896,19 @@ def test_f32_solves_without_a_schedule_fill_whole_waves(sfh, dims, tiles, stage)
         B.close()
     assert out[0][0] == out[1][0]
     assert np.array_equal(out[0][1], out[1][1])
+
+
+@pytest.mark.parametrize("dims,nrhs,flow", [((12, 12, 12, 12), 4, True), ((12, 12, 12, 12), 6, False),
+                                            ((12, 12, 12, 12), 5, False), ((16, 16, 16, 16), 2, True)])
+def test_fp64_dataflow_launch_serves_a_few_rounds_only(sfh, dims, nrhs, flow):
+    """FP64 batches whose hops would take the dataflow kernel more than four
+    rounds of a block's threads (more than three with more than four RHS) run
+    the per-phase kernels: the true residual either way."""
+    B = sfh.Batch([(dims, 0.3, nrhs)], precision="f64")
+    B.random_gauge(0, 0.5, 3)
+    for j in range(nrhs):
+        B.random_rhs(0, j, 4 + j)
+    B.solve(tol=1e-10)
+    assert (B.kernel_launches() == 2) == flow
+    assert max(B.true_residual(0, j) for j in range(nrhs)) < 1.5e-10
+    B.close()
