@@ -2189,10 +2189,7 @@ static cudaError_t flow_solve(CgWorkspace& w, const CgArgs& a, cudaStream_t stre
 // 183, FP32 277 -> 230, BF16 262 -> 232; 16^4 with 8 RHS FP16 28.6 -> 23.6; below
 // the line, 20^4 with 2 RHS, the lane lists would take 21.3 for 20.2.
 //
-// FP64: groups of two read a link once for both, but a block takes 1.6 times as
-// long as one of a single RHS, which tells where there are few waves: by the
-// waves of resident blocks (six systems of up to 10^4, 22 RHS, 20.9 -> 19.4 ms;
-// 16^4 with 4 RHS stays at two, 17.0 against 20.9).
+// FP64: f64_singles.
 //
 // One RHS, 16-bit storage: from 2000 tiles on the lane lists and two tiles an
 // item, from 6000 on four.  ms for two tiles with inline updates, lane lists
@@ -2215,18 +2212,46 @@ struct AutoSchedule {
     int nb1 = 0, nb2 = 0, tpi = 0, stage = 0;
 };
 
+// FP64: groups of two read a link once for both, but a block of two takes 1.35
+// times as long as one of a single RHS (odd RHS are groups of one in both),
+// which tells where there are few waves of resident blocks.  The waves are
+// counted as the lanes retire, heavier masses first: iterations go with 1 / m.
+// ms for groups of one and of two: 10^4 with 6 RHS (one wave each way) 3.9, 5.2;
+// 12^3 24 with 3 6.6, 7.5; 16^4 with 4 13.4, 10.9; 24^4 with 3 54.0, 49.2; six
+// systems of up to 10^4, 22 RHS of three masses, 19.4, 20.9.  Of 114 batches one takes
+// 1 % longer than with groups of two; on average 0.8 % are lost to the better
+// width of each (4.3 % with groups of two throughout).
+static bool f64_singles(const CgWorkspace& w)
+{
+    std::vector<double> masses;
+    for (const CgLane& L : w.lanes_h) masses.push_back(std::sqrt(L.m2));
+    std::sort(masses.rbegin(), masses.rend());
+    const double slots = (double)HopOcc<GP_F64_18, SP_F64, 2, true>::v * std::max(1, w.num_sms);
+    double singles = 0.0, twos = 0.0, from = 0.0;
+    for (double m : masses) {
+        const double until = 1.0 / std::max(m, 1e-3);
+        if (until <= from) continue;
+        std::vector<int> n(w.sys.size(), 0);  // lanes of either parity with at most this mass
+        for (const CgLane& L : w.lanes_h)
+            if (L.parity != 1 && std::sqrt(L.m2) <= m) n[L.sys] += 1;
+        double ones = 0.0, pairs = 0.0, odd = 0.0;
+        for (size_t k = 0; k < w.sys.size(); ++k) {
+            ones += 2.0 * w.sys[k].ntq * n[k];
+            pairs += 2.0 * w.sys[k].ntq * (n[k] / 2);
+            odd += 2.0 * w.sys[k].ntq * (n[k] & 1);
+        }
+        singles += (until - from) * std::ceil(ones / slots);
+        twos += (until - from) * std::ceil((pairs + odd) / slots) * (1.35 * pairs + odd) / (pairs + odd);
+        from = until;
+    }
+    return singles < twos;
+}
+
 static AutoSchedule auto_schedule(const CgWorkspace& w)
 {
     AutoSchedule s;
     if (w.prec == SFH_PREC_F64) {
-        // waves of resident blocks of groups of two (1.6 times as long) and of one
-        long b1 = 0, b2 = 0;
-        for (const CgSys& S : w.sys) {
-            b1 += 2L * S.ntq * S.nrhs;
-            b2 += 2L * S.ntq * ((S.nrhs + 1) / 2);
-        }
-        const long slots = (long)HopOcc<GP_F64_18, SP_F64, 2, true>::v * std::max(1, w.num_sms);
-        if (5 * ((b1 + slots - 1) / slots) < 8 * ((b2 + slots - 1) / slots)) s.nb1 = s.nb2 = 1;
+        if (f64_singles(w)) s.nb1 = s.nb2 = 1;
         return s;
     }
     const bool f16 = w.prec == SFH_PREC_F16, f32 = w.prec == SFH_PREC_F32;
