@@ -10,10 +10,6 @@ namespace sfh {
 
 namespace {
 
-// From here on the first copy repays the buffers (16 MB) and every copy its
-// threads; below, CUDA's own copy takes less than 8 ms.
-constexpr size_t kLeastBytes = (size_t)32 << 20;
-
 bool pageable(const void* host)
 {
     cudaPointerAttributes a;
@@ -132,14 +128,14 @@ cudaError_t HostCopy::move(char* dev, char* host, size_t bytes, int device, cuda
 
 cudaError_t HostCopy::in(void* dev, const void* host, size_t bytes, int device, cudaStream_t stream)
 {
-    if (bytes >= kLeastBytes && pageable(host) && !capturing(stream) && ready())
+    if (bytes >= CopyCredit::kLeast && pageable(host) && !capturing(stream) && credit_.enough(bytes, true) && ready())
         return pieces<true>((char*)dev, (char*)const_cast<void*>(host), bytes, device, stream);
     return cudaMemcpyAsync(dev, host, bytes, cudaMemcpyHostToDevice, stream);
 }
 
 cudaError_t HostCopy::out(void* host, const void* dev, size_t bytes, int device, cudaStream_t stream)
 {
-    if (bytes >= kLeastBytes && pageable(host) && !capturing(stream) && ready())
+    if (bytes >= CopyCredit::kLeast && pageable(host) && !capturing(stream) && credit_.enough(bytes, false) && ready())
         return pieces<false>((char*)const_cast<void*>(dev), (char*)host, bytes, device, stream);
     return cudaMemcpyAsync(host, dev, bytes, cudaMemcpyDeviceToHost, stream);
 }
