@@ -496,7 +496,9 @@ class Lattice:
 
     def set_schedule(self, width=0, tiles_per_block=0, stage_links=0):
         """Schedule of this lattice's mixed-precision solves (as
-        Batch.set_schedule; stage_links 3: one persistent launch per solve)."""
+        Batch.set_schedule; stage_links 3: one persistent launch per solve).  Any
+        but 0, 0, 0 keeps small solves, FP64 too, out of the dataflow launch,
+        which takes the GPU for itself: several threads solve faster then."""
         self._check(self.lib.sfh_set_schedule(self.h, width, tiles_per_block, int(stage_links)), "set_schedule")
 
     HMC_KERNELS = ("gauge_force", "fermion_force", "staples", "link_update", "stout_level", "stout_force",

@@ -2829,6 +2829,12 @@ static CgWorkspace* ctx_workspace(sfh_ctx* c, int prec, cudaError_t* err)
     return w;
 }
 
+// a context with a schedule of its own runs the per-phase kernels in FP64 too
+static FlowUse ctx_flow_use(const sfh_ctx* c)
+{
+    return c->sched_nb > 0 || c->sched_tpi > 0 || c->sched_stage != 0 ? FLOW_NEVER : FLOW_OPEN;
+}
+
 int ctx_solve_device(sfh_ctx* c, const void* b_eo, void* x_eo, double tol, int maxit, int prec,
                      sfh_cg_info* info)
 {
@@ -2849,9 +2855,9 @@ int ctx_solve_device(sfh_ctx* c, const void* b_eo, void* x_eo, double tol, int m
     size_t fs = (size_t)c->g.V * 6 * sizeof(double);
     e = cudaMemcpyAsync(w->rhs[0].b, b_eo, fs, cudaMemcpyDeviceToDevice, c->stream);
     if (e != cudaSuccess) return cuda_check(c, e, "cg rhs");
-    const bool lowp = prec != SFH_PREC_F64;  // the FP64 CG keeps the reference's schedule
+    const bool lowp = prec != SFH_PREC_F64;  // the FP64 CG keeps its own schedule
     e = workspace_solve(*w, tol, maxit, default_reliable_delta(prec), lowp ? c->sched_nb : 0, lowp ? c->sched_nb : 0,
-                        lowp ? c->sched_tpi : 0, lowp ? c->sched_stage : 0, c->stream);
+                        lowp ? c->sched_tpi : 0, lowp ? c->sched_stage : 0, c->stream, nullptr, ctx_flow_use(c));
     if (e != cudaSuccess) return cuda_check(c, e, "cg solve");
     if (w->timed_out) return set_error(c, SFH_ERR_TIMEOUT, "CG: a bounded device wait (grid barrier or neighbour staging) gave up");
     e = cudaMemcpyAsync(x_eo, w->rhs[0].xhi, fs, cudaMemcpyDeviceToDevice, c->stream);
@@ -2929,7 +2935,7 @@ int ctx_solve_pair_device(sfh_ctx* c, const void* const b_eo[2], void* const x_e
     w->auto_nb = lowp ? 1 : 0;
     const int nb = lowp ? c->sched_nb : 0;
     e = workspace_solve(*w, tol, maxit, default_reliable_delta(prec), nb, nb, lowp ? c->sched_tpi : 0,
-                        lowp ? c->sched_stage : 0, c->stream);
+                        lowp ? c->sched_stage : 0, c->stream, nullptr, ctx_flow_use(c));
     if (e != cudaSuccess) return cuda_check(c, e, "cg pair solve");
     if (w->timed_out) return set_error(c, SFH_ERR_TIMEOUT, "CG: a bounded device wait (grid barrier or neighbour staging) gave up");
     for (int k = 0; k < 2; ++k) {

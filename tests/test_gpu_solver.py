@@ -931,3 +931,31 @@ def test_fp64_group_widths_by_size_take_the_faster_one(sfh, dims, nrhs, width):
         best[schedule] = min(times[1:])
     B.close()
     assert best[(0, 0, 0)] < 1.05 * best[(width, 0, 0)], best
+
+
+def test_fp64_context_with_a_schedule_runs_the_per_phase_kernels(sfh, orc):
+    """A context's explicit schedule keeps its solves out of the dataflow
+    launch in FP64 too, where the schedule's numbers are the solver's own: the
+    solution is that of a full-lattice batch with a schedule, bit for bit, and
+    the oracle's residual; schedule 0, 0, 0 brings the dataflow launch back."""
+    dims, mass, tol = (8, 8, 8, 8), 0.1, 1e-10
+    U, b = orc.random_gauge(dims, 0.7, 61), orc.random_spinor(dims, 62)
+    B = sfh.Batch([(dims, mass, 1)], precision="f64", full_lattice=True)
+    B.set_gauge(0, U)
+    B.set_rhs(0, 0, b)
+    out = []
+    for schedule in ((1, 1, 0), (0, 0, 0)):
+        B.set_schedule(*schedule)
+        B.solve(tol=tol)
+        out.append(B.solution(0, 0))
+    assert B.kernel_launches() == 2
+    B.close()
+    assert not np.array_equal(out[0], out[1])  # else the comparison below shows nothing
+    lat = sfh.Lattice(dims, mass)
+    lat.upload_gauge(U)
+    for schedule, X in (((1, 1, 0), out[0]), ((0, 0, 0), out[1])):
+        lat.set_schedule(*schedule)
+        Y = lat.solve_CG_DDdagger(b, tol=tol, precision="f64")
+        assert np.array_equal(Y, X)
+        assert true_resid(orc, dims, mass, U, b, Y) < 1.5 * tol
+    lat.close()
