@@ -959,3 +959,57 @@ def test_fp64_context_with_a_schedule_runs_the_per_phase_kernels(sfh, orc):
         assert np.array_equal(Y, X)
         assert true_resid(orc, dims, mass, U, b, Y) < 1.5 * tol
     lat.close()
+
+
+@pytest.mark.parametrize("dims,masses,schedule", [
+    ((6, 4, 8, 6), [0.1], (1, 1, 0)),
+    ((8, 8, 8, 8), [0.1, 0.4], (1, 2, 0)),       # one RHS an item, two tiles
+    ((6, 10, 6, 10), [0.2, 0.05], (2, 1, 0)),    # both RHS in an item, the light one second
+    ((4, 4, 4, 8), [0.3, 0.1, 0.2], (2, 1, 0)),  # a group of two and one of one
+])
+def test_full_lattice_lanes_in_the_per_phase_kernels(sfh, orc, dims, masses, schedule):
+    """FP64 lanes over both parities (the reference's CG) in the per-phase
+    kernels, which larger lattices take: iterations and solutions against the
+    oracle's CG at each right-hand side's own mass, and against the dataflow
+    launch that lattices of this size take without a schedule."""
+    tol = 1e-10
+    U = orc.random_gauge(dims, 0.6, 71)
+    bs = [orc.random_spinor(dims, 72 + j) for j in range(len(masses))]
+    B = sfh.Batch([(dims, masses[0], len(masses))], precision="f64", full_lattice=True)
+    B.set_gauge(0, U)
+    for j, (b, m) in enumerate(zip(bs, masses)):
+        B.set_rhs(0, j, b)
+        B.set_rhs_mass(0, j, m)
+    for s in (schedule, (0, 0, 0)):
+        B.set_schedule(*s)
+        B.solve(tol=tol)
+        assert (B.kernel_launches() == 2) == (s == (0, 0, 0))
+        for j, (b, m) in enumerate(zip(bs, masses)):
+            X, it, _, st = orc.cg(dims, m, U, b, tol)
+            info = B.info(0, j)
+            assert st == 0 and info["status"] == 0 and abs(info["iters"] - it) <= 1
+            # two solutions of residual tol (one iteration apart at most)
+            assert np.linalg.norm(B.solution(0, j) - X) <= 2 * tol * (m ** 2 + 16) / m ** 2 * np.linalg.norm(X)
+            assert true_resid(orc, dims, m, U, b, B.solution(0, j)) < 1.5 * tol
+    B.close()
+
+
+@pytest.mark.parametrize("precision", ["f64", "f32", "f16"])
+def test_timed_solve_runs_the_schedule_of_the_graph_solve(sfh, precision):
+    """With a schedule set, the timed solve launches the kernels of the graph
+    solve one by one: the same solutions bit for bit, and every iteration's
+    kernels timed."""
+    B = sfh.Batch([((4, 4, 4, 8), 0.1, 3), ((6, 6, 6, 6), 0.2, 2)], precision=precision)
+    B.set_schedule(2, 1, 0)
+    for k, n in ((0, 3), (1, 2)):
+        B.random_gauge(k, 0.5, 7 + k)
+        for j in range(n):
+            B.random_rhs(k, j, 17 + 10 * k + j)
+    out = []
+    for timed in (False, True):
+        times = B.solve_timed(tol=1e-10) if timed else B.solve(tol=1e-10)
+        assert timed or B.kernel_launches() > 2
+        out.append([B.solution(k, j) for k, n in ((0, 3), (1, 2)) for j in range(n)])
+    assert all(np.array_equal(a, b) for a, b in zip(*out))
+    assert times["cg_hop1"][1] == times["cg_hop2"][1] == times["cg_update"][1] > 0
+    B.close()
