@@ -60,8 +60,6 @@ namespace sfh {
 
 namespace {
 
-
-
 // resident 256-thread blocks per SM the hop kernels are compiled for (at most
 // 85 registers a thread for three, 64 for four): up to two lanes a block fit
 // three blocks, four with FP16 links and vectors (their packed-half products

@@ -602,11 +602,12 @@ template <int SP> struct FlowMax {
     static constexpr int threads = SP == SP_F64 ? 256 : 512;
 };
 
-// ONE: every thread has one piece of a hop, whose neighbours and links it
-// keeps in registers for the whole solve.
-template <int GP, int SP, int SPL, bool ONE>
+// Four threads a site: every thread has one piece of a hop (ONE; flow_plan), whose
+// neighbours and links it keeps in registers for the whole solve.
+template <int GP, int SP, int SPL>
 __global__ void __launch_bounds__(FlowMax<SP>::threads, 1) cg_flow(CgArgs a, FlowArgs f)
 {
+    constexpr bool ONE = SPL == 4;
     typedef typename GaugeFmt<GP>::R R;
     typedef typename SpinorFmt<SP>::R RS;
     typedef FlowVec<SP> F;
@@ -1053,7 +1054,6 @@ bool flow_plan(const std::vector<CgSys>& sys, int prec, int num_sms, FlowPlan* p
     const int all = warps(plan->split);
     plan->rounds = (64 * all + most - 1) / most;
     plan->threads = 64 * ((all + plan->rounds - 1) / plan->rounds);
-    plan->one = plan->rounds == 1;
     if (plan->dyn > kFlowMaxSmem) return false;
     // FP64 serves the RHS of a block one after the other, round by round, where
     // the per-phase kernels take a link for two: from five rounds on, with more
@@ -1079,20 +1079,21 @@ bool flow_beats_tuned(const std::vector<CgSys>& sys, const FlowPlan& plan)
 cudaError_t flow_launch(int prec, const CgArgs& a, const FlowArgs& f, const FlowPlan& plan, cudaStream_t stream)
 {
     typedef void (*Kernel)(CgArgs, FlowArgs);
-    // links in registers only where a thread has one direction: 18 to 72 of
-    // its 128 or 255 (a hop of 8^3 16 in FP32 2700 cycles against 4200)
-    const int sl = plan.split == 4 ? (plan.one ? 3 : 2) : plan.split - 1;
-    static const Kernel f64[4] = {cg_flow<GP_F64_18, SP_F64, 1, false>, cg_flow<GP_F64_18, SP_F64, 2, false>,
-                                  cg_flow<GP_F64_18, SP_F64, 4, false>, cg_flow<GP_F64_18, SP_F64, 4, true>};
-    static const Kernel f32[4] = {cg_flow<GP_F32_12, SP_F32, 1, false>, cg_flow<GP_F32_12, SP_F32, 2, false>,
-                                  cg_flow<GP_F32_12, SP_F32, 4, false>, cg_flow<GP_F32_12, SP_F32, 4, true>};
-    static const Kernel f16[4] = {cg_flow<GP_F16_12, SP_F16, 1, false>, cg_flow<GP_F16_12, SP_F16, 2, false>,
-                                  cg_flow<GP_F16_12, SP_F16, 4, false>, cg_flow<GP_F16_12, SP_F16, 4, true>};
+    // links in registers only where a thread has one direction (four threads a
+    // site): 18 to 72 of its 128 or 255 (a hop of 8^3 16 in FP32 2700 cycles
+    // against 4200)
+    const int sl = plan.split / 2;
+    static const Kernel f64[3] = {cg_flow<GP_F64_18, SP_F64, 1>, cg_flow<GP_F64_18, SP_F64, 2>,
+                                  cg_flow<GP_F64_18, SP_F64, 4>};
+    static const Kernel f32[3] = {cg_flow<GP_F32_12, SP_F32, 1>, cg_flow<GP_F32_12, SP_F32, 2>,
+                                  cg_flow<GP_F32_12, SP_F32, 4>};
+    static const Kernel f16[3] = {cg_flow<GP_F16_12, SP_F16, 1>, cg_flow<GP_F16_12, SP_F16, 2>,
+                                  cg_flow<GP_F16_12, SP_F16, 4>};
     const Kernel k = prec == SFH_PREC_F64      ? f64[sl]
                      : prec == SFH_PREC_F32    ? f32[sl]
                      : prec == SFH_PREC_F16    ? f16[sl]
-                     : prec == SFH_PREC_F32_18 ? cg_flow<GP_F32_18, SP_F32, 1, false>
-                                               : cg_flow<GP_BF16_12, SP_BF16, 1, false>;
+                     : prec == SFH_PREC_F32_18 ? cg_flow<GP_F32_18, SP_F32, 1>
+                                               : cg_flow<GP_BF16_12, SP_BF16, 1>;
     // the same limit from every handle: it belongs to the kernel, and another
     // thread may be about to launch it with more than this plan takes
     cudaError_t e = cudaFuncSetAttribute((const void*)k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kFlowMaxSmem);

@@ -21,7 +21,9 @@ struct FlowTeam {
 struct FlowArgs {
     const FlowTeam* teams;
     const int* blk_team;        // team of every block
-    uint4* sums;                // per team [2][nblk][4 nlanes] {double, tag}
+    // {double, tag} words per team [2][4 nlanes][nblk], the block fastest, each
+    // half followed by the totals' copies [ceil(nblk / 8)][4 nlanes]
+    uint4* sums;
     unsigned* flags;            // one per block: barriers passed
     char* const* pub;           // per RHS: published p, then published t
     int* err;                   // set by a wait that gave up
@@ -36,8 +38,7 @@ struct FlowPlan {
     size_t words = 0, pub_bytes = 0;
     int threads = 0;
     int split = 1;                 // threads per site in a hop
-    int rounds = 1;                // of the block's threads, for a hop
-    bool one = false;              // rounds == 1
+    int rounds = 1;                // of the block's threads, for a hop (1 where split is 4)
     size_t dyn = 0;                // dynamic shared memory of a block
 };
 // false where the per-phase kernels are the better ones (or the systems do
