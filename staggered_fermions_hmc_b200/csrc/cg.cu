@@ -2211,14 +2211,15 @@ struct AutoSchedule {
 };
 
 // FP64: groups of two read a link once for both, but a block of two takes 1.35
-// times as long as one of a single RHS (odd RHS are groups of one in both),
-// which tells where there are few waves of resident blocks.  The waves are
+// times as long as one of a single RHS, and with one lane (the odd RHS, or one
+// left by a heavier mass) still 1.1 times, which tells where there are few waves
+// of resident blocks.  The waves are
 // counted as the lanes retire, heavier masses first: iterations go with 1 / m.
 // ms for groups of one and of two: 10^4 with 6 RHS (one wave each way) 3.9, 5.2;
 // 12^3 24 with 3 6.6, 7.5; 16^4 with 4 13.4, 10.9; 24^4 with 3 54.0, 49.2; six
-// systems of up to 10^4, 22 RHS of three masses, 19.4, 20.9.  Of 114 batches one takes
-// 1 % longer than with groups of two; on average 0.8 % are lost to the better
-// width of each (4.3 % with groups of two throughout).
+// systems of up to 10^4, 22 RHS of three masses, 19.4, 20.9.  Of 114 batches two take
+// 4 and 5 % longer than with groups of two; on average 0.6 % are lost to the
+// better width of each (4.3 % with groups of two throughout).
 static bool f64_singles(const CgWorkspace& w)
 {
     std::vector<double> masses;
@@ -2239,7 +2240,7 @@ static bool f64_singles(const CgWorkspace& w)
             odd += 2.0 * w.sys[k].ntq * (n[k] & 1);
         }
         singles += (until - from) * std::ceil(ones / slots);
-        twos += (until - from) * std::ceil((pairs + odd) / slots) * (1.35 * pairs + odd) / (pairs + odd);
+        twos += (until - from) * std::ceil((pairs + odd) / slots) * (1.35 * pairs + 1.1 * odd) / (pairs + odd);
         from = until;
     }
     return singles < twos;

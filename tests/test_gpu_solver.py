@@ -1013,3 +1013,22 @@ def test_timed_solve_runs_the_schedule_of_the_graph_solve(sfh, precision):
     assert all(np.array_equal(a, b) for a, b in zip(*out))
     assert times["cg_hop1"][1] == times["cg_hop2"][1] == times["cg_update"][1] > 0
     B.close()
+
+
+def test_fp64_pair_of_masses_takes_single_groups_where_one_lane_is_left(sfh):
+    """Two masses on the same links, the heavy one done after a third of the
+    iterations: a group of two then runs with one lane, 1.1 times as long as a
+    group of one, so that groups of one are the faster ones here by 5 % over
+    the solve (device times, the best of four solves; half of that is the
+    bound)."""
+    B = sfh.Batch([((16, 16, 16, 24), 0.1, 2)], precision="f64", full_lattice=True)
+    B.set_rhs_mass(0, 1, 0.3)
+    B.random_gauge(0, 0.3, 3)
+    for j in range(2):
+        B.random_rhs(0, j, 4 + j)
+    best = {}
+    for schedule in ((0, 0, 0), (1, 0, 0)):
+        B.set_schedule(*schedule)
+        best[schedule] = min(sum(t[0] for t in B.solve_timed(tol=1e-10).values()) for _ in range(5))
+    B.close()
+    assert best[(0, 0, 0)] < 1.025 * best[(1, 0, 0)], best
