@@ -607,22 +607,27 @@ def run_extras(sfh, hbm, quick=False):
 # ---------------------------------------------------------------------------
 # C5: full HMC on 24^4 (bench.py --workload c5)
 # ---------------------------------------------------------------------------
-# algorithmic bytes and flops per link of the HMC kernels (FP64 links 144 B,
-# momenta 144 B, spinors 48 B per site = 24 B per link of the site):
-#   gauge force + kick   U in, P in and out; 84 staple matmuls + U V, 198 flop each
-#   fermion force + kick U, X, Y in, P in and out; two outer products and matmuls
-#   staples              U in, A1 and A2 out; 84 matmuls
-#   link update          U in and out, P in; exp(iQ) and one matmul
-#   stout level          U in, U' out; 12 plaquette-staple matmuls, exp, one matmul
-#   action, plaquette    U in; 84 / 12 staple matmuls and the traces
+# bytes that each HMC kernel cannot do without and flops that it does, per
+# link (FP64 links 144 B, momenta 144 B, spinors 48 B per site = 24 B per link
+# of the site; a product of 3x3 complex matrices 198 flop, the real trace of
+# one 36):
+#   gauge force + kick   U in, P in and out; six sides of 11 products, U V
+#   fermion force + kick U, X, Y in, P in and out; a product, a matrix on a
+#                        vector, two outer products, two differences
+#   staples              U in, A1 and A2 out; six sides of 12 products
+#   link update          U in and out, P in; Q^2, tr Q^3, the exponential, E U
+#   stout level          U in, U' out; 12 staple products, C U^dag, Q^2, E U
+#   action, plaquette    U in; per site and plane 8 products and 3 traces, or
+#                        2 and 1 (six planes for four links)
+MATRIX_FLOPS, TRACE_FLOPS, EXP_FLOPS = 198, 36, 200
 HMC_KERNEL_COST = {  # (bytes, flops) per link
-    "gauge_force": (3 * 144, 85 * 198),
-    "fermion_force": (3 * 144 + 2 * 24, 4 * 198),
-    "staples": (3 * 144, 84 * 198),
-    "link_update": (3 * 144, 3 * 198 + 200),
-    "stout_level": (2 * 144, 14 * 198 + 200),
-    "action": (144, 85 * 198),
-    "plaquette": (144, 13 * 198),
+    "gauge_force": (3 * 144, (6 * 11 + 1) * MATRIX_FLOPS),
+    "fermion_force": (3 * 144 + 2 * 24, MATRIX_FLOPS + 66 + 2 * 54 + 2 * 18),
+    "staples": (3 * 144, 6 * 12 * MATRIX_FLOPS),
+    "link_update": (3 * 144, 2 * MATRIX_FLOPS + 2 * TRACE_FLOPS + EXP_FLOPS),
+    "stout_level": (2 * 144, 15 * MATRIX_FLOPS + 2 * TRACE_FLOPS + EXP_FLOPS),
+    "action": (144, 1.5 * (8 * MATRIX_FLOPS + 3 * TRACE_FLOPS)),
+    "plaquette": (144, 1.5 * (2 * MATRIX_FLOPS + TRACE_FLOPS)),
 }
 FP64_TFLOPS_NOMINAL = 40.0  # B200 datasheet FP64 (no measured FP64 peak on this pool)
 HBM_SPEC_GBS = 8000.0  # B200 datasheet HBM3e bandwidth; fractions of it are reported beside the measured ones
@@ -642,7 +647,8 @@ def hmc_kernel_table(lat, hbm):
             tfs = f * nlinks / (ms * 1e-3) / 1e12
             row.update({"GB/s": gbs, "frac_hbm": gbs / hbm, "TFLOP/s_fp64": tfs,
                         "frac_fp64_nominal": tfs / FP64_TFLOPS_NOMINAL,
-                        "bound": "fp64" if f / b > FP64_TFLOPS_NOMINAL * 1e3 / hbm else "hbm"})
+                        # the lower roof at these bytes and flops, not what is reached
+                        "roof": "fp64" if f / b > FP64_TFLOPS_NOMINAL * 1e3 / hbm else "hbm"})
         out[name] = row
     return out
 

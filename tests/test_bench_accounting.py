@@ -235,3 +235,37 @@ def test_e2e_pipeline_reraises_a_side_thread_error():
     with pytest.raises(RuntimeError, match="upload failed"):
         bench.e2e_pipelined(fake_torch, (FakeBatch("A"), FakeBatch("B")), upload, lambda X: None, 4)
     assert solves == ["A", "B", "A"]  # the step whose side thread failed still finished its solve
+
+
+def test_hmc_kernel_flops_are_those_of_the_kernels():
+    """The flops per link that the C5 table counts are the matrix products and
+    traces which the staple sides and the plane loops of csrc/gauge.cu form
+    (walking every path on its own, as the reference does, would take 84 and
+    85 products a link)."""
+    import re
+
+    import bench
+    src = open(os.path.join(ROOT, "staggered_fermions_hmc_b200", "csrc", "gauge.cu")).read()
+
+    def body(name):
+        return re.search(r"\n(?:__device__ __forceinline__ )?void " + name + r"\(.*?\n\}\n|"
+                         r"\n__device__ __forceinline__ void " + name + r"\(.*?\n\}\n", src, re.S).group(0)
+
+    def products(text):
+        return len(re.findall(r"\bm3_(?:mul|mul_adj|adj_mul|mul_to<true>)\(", text))
+
+    side = body("staple_side")
+    pair = r"if constexpr \(SPLIT\) \{(.*?)\n    \} else \{(.*?)\n    \}"
+    assert len(re.findall(pair, side, re.S)) == 2
+    one = products(re.sub(pair, r"\2", side, flags=re.S))
+    split = products(re.sub(pair, r"\1", side, flags=re.S))
+    loops = body("plane_loops")
+    plaq, rect = re.split(r"if constexpr \(RECT\)", loops)
+    M, T = 198, 36
+    cost = {k: f for k, (b, f) in bench.HMC_KERNEL_COST.items()}
+    assert (one, split) == (11, 12)
+    assert cost["gauge_force"] == (6 * one + 1) * M
+    assert cost["staples"] == 6 * split * M
+    traces = [len(re.findall(r"m3_retr_adj\(", t)) for t in (plaq, rect)]
+    assert cost["plaquette"] == 1.5 * (products(plaq) * M + traces[0] * T)
+    assert cost["action"] == 1.5 * ((products(plaq) + products(rect)) * M + sum(traces) * T)
