@@ -357,9 +357,10 @@ int sfh_batch_autotune(sfh_batch* batch, int probe_iters, int* best_width);
  * block of the iteration kernels (0 = 2, or 1 where two would give the first
  * hop fewer than four work items per SM), and the hop kernels' link staging
  * (width, tiles and staging all 0, the default: small batches, at most 8 RHS
- * per system and 1024 site-lanes per SM and parity, fewer for the wider
- * precisions, run the whole solve in one dataflow launch, whose sums are added
- * in another order; the rest take a schedule by their size):
+ * per system and 1024 site-lanes per SM and parity (FP32 about 830, FP64 470 to
+ * 510, with more than four RHS 220 to 380), run the whole solve in one dataflow
+ * launch, whose sums are added in another order; the rest take a schedule by
+ * their size):
  * 0 links read directly per RHS group; 1 staged in shared memory per work
  * item with asynchronous copies; 2 system-blocked: one block per tile serves
  * every RHS of its system in groups of the RHS-block width, the tile's links

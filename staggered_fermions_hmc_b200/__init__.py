@@ -529,7 +529,7 @@ class Lattice:
 
 class Batch:
     """Many independent D D^dag solves (lattices, masses, right-hand sides)
-    solved by one persistent launch.  No reference counterpart."""
+    that advance together.  No reference counterpart."""
 
     def __init__(self, systems, precision="f32", full_lattice=False, device=0):
         self.lib = load_library()

@@ -68,10 +68,12 @@ namespace {
 // registers and two
 template <int GP, int SP, int NB, bool SUMS, bool RUI = true> struct HopOcc {
     // without the inline FP64 reliable-update hop the kernels need fewer
-    // registers: FP16 fits in 48 (five blocks), the FP32-arithmetic ones with
+    // registers: FP16 runs in 48 (five blocks; the second hop spills 48 / 48
+    // bytes with one RHS and 124 / 112 with two, the first with its prefetch
+    // 36 / 40 and 192 / 228, see PF), the FP32-arithmetic ones with
     // 12-real links in 64 (four); 18-real FP32 links keep three.  FP16 in
     // groups of four RHS: the first hop fits in 64 registers (four blocks,
-    // no spills), the second, with its sums, in 80 (three)
+    // no spills), the second, with its sums, takes 80 (three; 120 / 88 spilled)
     static constexpr int v = (NB == 4 && GP == GP_F16_12 && SP == SP_F16 && !RUI) ? (SUMS ? 3 : 4)
                              : (SP == SP_F64 || NB > 2) ? 2
                              : ((GP == GP_F16_12 && SP == SP_F16) ? (RUI ? 4 : 5)
@@ -238,9 +240,11 @@ __device__ __forceinline__ void prefetch_link(const void* Ulo, int p, int mu, in
 // sn + l * W where it holds them (tstage.cuh), else from global memory.
 // PF (FP16): the next direction's links are brought into the L1 meanwhile.
 // Worth its instructions only in the first hop with one or two RHS and no
-// inline reliable updates, where registers are left: 32^3 64, 99 -> 90 us a
-// launch, the solve 56.7 -> 55.5 ms; 24^3 48 with two, 48.3 -> 44.6 us (the
-// vectors too: 92 us; with four RHS 75 -> 97; the second hop spills, 120 -> 123).
+// inline reliable updates: 32^3 64, 99 -> 90 us a launch, the solve 56.7 -> 55.5
+// ms; 24^3 48 with two, 48.3 -> 44.6 us (the vectors too: 92 us; with four RHS 75
+// -> 97; the second hop 120 -> 123).  The gain is net of a spill: without it the
+// kernel needs 45 of its 48 registers, with its six addresses 36 / 40 bytes
+// (stores / loads) go to the stack with one RHS and 192 / 228 with two.
 template <int GP, int SP, int NB, bool STG, bool COH = false, bool NST = false, bool PF = false>
 __device__ __forceinline__ void hop_lanes(const void* Ulo, const typename GaugeFmt<GP>::E* sl, const Nbr& n, int q,
                                           int i, int Vh, const void* const (&in)[NB], const bool (&on)[NB],
@@ -2255,7 +2259,12 @@ static AutoSchedule auto_schedule(const CgWorkspace& w)
     }
     const bool f16 = w.prec == SFH_PREC_F16, f32 = w.prec == SFH_PREC_F32;
     if (w.nlanes > 2) {
-        if (w.auto_nb > 0) return s;  // a pair of masses keeps its own widths
+        // A pair of masses keeps groups of one and the default tiles.  The rule
+        // for its light lane alone would be as fast at 24^4 in FP32 (two steps of
+        // a trajectory 286.4 ms, 285.8 with it) and faster at 20^3 32 (268, 241)
+        // and 24^3 32 (424, 366); FP16 with lane lists 241, 230 at 24^4 and 343,
+        // 340 at 24^3 32.
+        if (w.auto_nb > 0) return s;
         long work = 0;
         int most = 1;
         for (const CgSys& S : w.sys) {

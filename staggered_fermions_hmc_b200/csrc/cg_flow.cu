@@ -992,11 +992,16 @@ static size_t block_bytes(int prec, int n, int nrhs)
     return (size_t)2 * n * (nrhs * 4 * (sp == SP_F64 ? 48 : (sp == SP_F32 ? 24 : 16)) + 4 * sizeof(NbrPair));
 }
 
-constexpr size_t kFlowMaxSmem = 208 * 1024;  // what is left of the SM's 256 KB caches the links
+// 208 of the 227 KB that a block may have: up to 6 go to its other arrays, and
+// what the SM has left caches the links.  With one RHS FP32 meets this line at
+// 832 sites, where the per-phase kernels catch up (20^3 30, 811 sites, 10.7 ms;
+// 20^3 32, 865 sites, by these 11.7), and FP64 at 474 (16^3 32, 443 sites, 10.7
+// ms either way); the 16-bit formats and several RHS in FP64 meet others first.
+constexpr size_t kFlowMaxSmem = 208 * 1024;
 // Checkerboard sites per parity and block: at least 32, so that a warp's
 // words are whole lines (4^4 in one block 7.3 us, in four 5.9); site-lanes at
 // most 1024, where the per-phase kernels catch up (FP16 at 886: 50 us against
-// 54; FP64 runs out of shared memory before, at 475: 53 against 58 at 443).
+// 54; FP64 at 443: 53 against 58).
 constexpr int kFlowMinSites = 32;
 constexpr int kFlowMaxSiteLanes = 1024;
 

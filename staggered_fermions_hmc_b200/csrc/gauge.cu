@@ -19,8 +19,8 @@
 // force 363 -> 228 us at 16^4, 2196 -> 1160 us at 24^4 (1399 with the directions
 // of a site far apart in the grid, 1242 with the links loaded as read-only
 // data); staples 2470 -> 1300 us; a heatbath sweep 3.57 -> 0.60 ms at 16^4, 18.1 ->
-// 3.3 ms at 24^4.  It runs at 17 TFLOP/s, 0.48 of the FP64 pipe, latency bound on
-// 12 warps per SM (168 registers): a third of the stalls are link loads, a
+// 3.3 ms at 24^4.  It runs at 15 TFLOP/s (198 a product), 0.38 of the FP64 pipe,
+// latency bound on 12 warps per SM (168 registers): a third of the stalls are link loads, a
 // fifth each FMA latency and instruction fetch.  A row of the staples per thread (80 registers, 24
 // warps, every link read by three threads) was bound by the L1: 2696 us.
 #include "sfh_internal.h"
