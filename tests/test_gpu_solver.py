@@ -918,17 +918,18 @@ def test_fp64_dataflow_launch_serves_a_few_rounds_only(sfh, dims, nrhs, flow):
 def test_fp64_group_widths_by_size_take_the_faster_one(sfh, dims, nrhs, width):
     """FP64 batches above the dataflow launch's sizes without a schedule take
     groups of one or two right-hand sides: here the other width takes 1.1 to
-    1.2 times as long (device times of the iteration kernels, the best of
-    three solves), so half of that is the bound."""
+    1.2 times as long (device times of the iteration kernels, the best of six
+    solves taken in turn), so half of that is the bound."""
     best = {}
     B = sfh.Batch([(dims, 0.3, nrhs)], precision="f64")
     B.random_gauge(0, 0.5, 3)
     for j in range(nrhs):
         B.random_rhs(0, j, 4 + j)
-    for schedule in ((0, 0, 0), (width, 0, 0)):
-        B.set_schedule(*schedule)
-        times = [sum(t[0] for t in B.solve_timed(tol=1e-10).values()) for _ in range(4)]
-        best[schedule] = min(times[1:])
+    for _ in range(6):
+        for schedule in ((0, 0, 0), (width, 0, 0)):
+            B.set_schedule(*schedule)
+            ms = sum(t[0] for t in B.solve_timed(tol=1e-10).values())
+            best[schedule] = min(ms, best.get(schedule, ms))
     B.close()
     assert best[(0, 0, 0)] < 1.05 * best[(width, 0, 0)], best
 
@@ -1019,16 +1020,18 @@ def test_fp64_pair_of_masses_takes_single_groups_where_one_lane_is_left(sfh):
     """Two masses on the same links, the heavy one done after a third of the
     iterations: a group of two then runs with one lane, 1.1 times as long as a
     group of one, so that groups of one are the faster ones here by 5 % over
-    the solve (device times, the best of four solves; half of that is the
-    bound)."""
+    the solve (device times, the best of six solves taken in turn; half of that
+    is the bound)."""
     B = sfh.Batch([((16, 16, 16, 24), 0.1, 2)], precision="f64", full_lattice=True)
     B.set_rhs_mass(0, 1, 0.3)
     B.random_gauge(0, 0.3, 3)
     for j in range(2):
         B.random_rhs(0, j, 4 + j)
     best = {}
-    for schedule in ((0, 0, 0), (1, 0, 0)):
-        B.set_schedule(*schedule)
-        best[schedule] = min(sum(t[0] for t in B.solve_timed(tol=1e-10).values()) for _ in range(5))
+    for _ in range(6):
+        for schedule in ((0, 0, 0), (1, 0, 0)):
+            B.set_schedule(*schedule)
+            ms = sum(t[0] for t in B.solve_timed(tol=1e-10).values())
+            best[schedule] = min(ms, best.get(schedule, ms))
     B.close()
     assert best[(0, 0, 0)] < 1.025 * best[(1, 0, 0)], best
